@@ -2094,6 +2094,17 @@ static int launch_shaped(SelectParams& p, const AttendRequest& ar, int n_pairs, 
 }
 
 
+// Pages a pair of the one-kernel step attends, as far as the host can tell: k picked blocks, or under the epsilon
+// rule a sixteenth of them (what ia_suggest_splits assumes).  0: the step will not run as one kernel.
+template <typename T, int D, int G>
+static int fused_step_pages(const SelectParams& p, const AttendRequest& ar, int max_tiles) {
+  if (!(sizeof(T) == 2 && D == 128 && G <= 8) || ar.req == nullptr || p.xch.n_ranks > 0 ||
+      ar.geom->n_pool_pages <= 0 || !fused_step_enabled())
+    return 0;
+  const int blocks = p.mode == IA_SELECT_TOPK ? min(p.top_k, p.max_blocks) : max_tiles * kTileBlocks / 16;
+  return blocks * (p.block_size / 16);
+}
+
 template <typename T, int D, int G, typename KB, int BOUND>
 static int launch_typed(const SelectParams& base, const AttendRequest& ar, int n_pairs, cudaStream_t stream) {
   constexpr bool DIAG = BOUND == 1, PACKED = BOUND == 2;
@@ -2121,6 +2132,15 @@ static int launch_typed(const SelectParams& base, const AttendRequest& ar, int n
   const int n_cand = xch_on ? p.xch.n_ranks * p.max_sel : 0;
   int cluster = 1;
   while (cluster < 8 && n_pairs * cluster * 2 <= sms && max_tiles / (cluster * 2) >= 2) cluster *= 2;
+  // One-kernel step: the cluster also shares the pair's pages, and one SM pulls only about 46 GB/s (0.18 us per
+  // 8 KB page), so with few pairs it is the attention that wants the larger cluster, however few tiles there are
+  // to score.  A further doubling costs about 1.5 us (wider cluster barriers, one more share to merge) and takes
+  // off as many pages as it leaves per CTA: the line is drawn at 16.  8 pairs x 256 pages (Llama-3-8B, one
+  // sequence, top-64 of 110 blocks), clusters of 2 / 4 / 8: 47 / 40 / 36 us (four-layer decode step 783 / 758 / 738 us).  128 CTAs at most: a GPC holds two
+  // clusters of 8 with one CTA per SM, a 17th would run alone in a second wave.
+  if (const int pages = fused_step_pages<T, D, G>(p, ar, max_tiles); pages > 0)
+    while (cluster < 8 && n_pairs * cluster * 2 <= (cluster == 4 ? min(sms, 128) : sms) && pages / (cluster * 2) >= 16)
+      cluster *= 2;
   if (const char* force = getenv("INTERATTN_B200_SELECT_CLUSTER")) {
     const int c = atoi(force);
     if (c == 1 || c == 2 || c == 4 || c == 8) cluster = c;

@@ -131,6 +131,37 @@ def test_fused_step_with_epsilon_rule(monkeypatch):
     _check_against_oracle(cfg, case, summ, out, idx, cnt)
 
 
+@pytest.mark.parametrize("rep_mode", ["sparse_only", "hybrid"])
+@pytest.mark.parametrize("batch,hkv,group,n_blocks,top_k", [
+    (1, 1, 1, 40, 32),   # one pair, 128 pages: the largest cluster, one query row
+    (1, 8, 4, 110, 64),  # eight pairs, four tiles of blocks for eight CTAs: half of them score nothing
+    (2, 8, 8, 33, 16),   # 128 CTAs, 64 pages: clusters end where a CTA would get fewer than 16
+    (2, 9, 2, 70, 64),   # 18 pairs x 8 = 144 CTAs fit the SMs, but not as clusters of eight
+    (3, 8, 4, 20, 3),    # too few pages to widen the cluster
+])
+def test_cluster_chosen_for_few_pairs(batch, hkv, group, n_blocks, top_k, rep_mode, monkeypatch):
+    """The launcher's own cluster size (nothing pinned) against one CTA per pair: the same blocks, and outputs that
+    differ by the merge order of the shares only (fp32 sums: far below the bf16 rounding of the output)."""
+    ops = _ops()
+    cfg = DecodeConfig("few_pairs", "bfloat16", batch, hkv * group, hkv, 128, 16, 64, top_k,
+                       tuple(n_blocks * 64 - 5 - 64 * b for b in range(batch)), (19,) * batch, seed=21)
+    case = make_case(cfg, spare_pages=3)
+    q, kv = to_device(case)
+    summ = ops.build_summaries(kv, cfg.block_size, max_blocks=max_blocks_of(case))
+    got = []
+    for cluster in (None, "1"):
+        if cluster is not None:
+            monkeypatch.setenv("INTERATTN_B200_SELECT_CLUSTER", cluster)
+        step = ops.DecodeAttention(kv, summ, cfg.n_q_heads, top_k=top_k, rep_mode=rep_mode)
+        out = step.step(q).clone()
+        torch.cuda.synchronize()
+        assert ops.last_decode_fused() and ops.device_status() == 0
+        got.append((out.float(), step.sel_idx.clone(), step.sel_count.clone()))
+    assert torch.equal(got[0][1], got[1][1]) and torch.equal(got[0][2], got[1][2])
+    # two bf16 ulps of the value: P is rounded to bf16 relative to the running maximum of its own warp
+    torch.testing.assert_close(got[0][0], got[1][0], rtol=2 ** -7, atol=2 ** -7)
+
+
 @pytest.mark.parametrize("cluster", [1, 2])
 def test_fused_step_with_more_pages_than_the_page_list_holds(cluster, monkeypatch):
     """One query row per kv head and an epsilon below every score: all blocks are kept, four pages each -
