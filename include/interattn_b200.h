@@ -23,6 +23,8 @@
  *   ia_finalize         <- _condition_block_stage2_reduce_kernel IMPL/legacy.py:765-794
  *   ia_decode_attention <- _condition_block_decode_output_fused_triton
  *                            IMPL/core.py:1035-1155 (the launches of one layer-step)
+ *   ia_build_prompt_blocks <- _build_prompt_blocks, the whole dict of one sequence over a
+ *                          contiguous cache                   IMPL/core.py:449-500
  *   ia_update_summaries <- no counterpart (the reference never re-blocks its suffix)
  *   ia_select_split, ia_sparse_decode_exchange, ia_finalize_exchange, ia_finalize_gathered
  *                       <- no counterpart (split-KV across GPUs; the reference has one GPU)
@@ -181,6 +183,32 @@ int ia_build_summaries(const void* k_pool, const void* v_pool, const int32_t* bl
 int ia_update_summaries(const void* k_pool, const void* v_pool, const int32_t* block_table,
                         const int32_t* prefix_lens, const int32_t* first_blocks, const ia_geom* geom,
                         const ia_summaries* out, ia_stream_t stream);
+
+/* What _build_prompt_blocks returns next to the summaries (all device memory, written by the call). */
+typedef struct ia_prompt_extras {
+  float* v_bar_f32;      /* [n_kv_heads, n_blocks, head_dim] fp32 copies of the stored values; null: not wanted */
+  float* k_max_f32;
+  float* k_min_f32;
+  void* k_block;         /* [n_kv_heads, n_blocks, block_size, head_dim] KV dtype, rows past `length` zero; */
+  void* v_block;         /* both or neither; null: not wanted */
+  int64_t* token_idx;    /* [n_blocks * block_size] 0, 1, 2, ... */
+  uint8_t* valid_token;  /* [n_blocks * block_size] 1 where token_idx < length */
+  int64_t* counts;       /* [n_blocks] tokens of each block */
+  float* v_norm_all;     /* [n_kv_heads] max of v_norm_max over the blocks */
+  int32_t* table;        /* [table_entries] identity block table */
+  int32_t* prefix_len;   /* one entry each: length */
+  int32_t* seq_len;
+  int32_t table_entries;
+  int32_t reserved;      /* 0 */
+} ia_prompt_extras;
+
+/* The reference's _build_prompt_blocks for one sequence whose `length` tokens lie contiguously:
+ * token t of head h at k + h * geom->pool_head_stride + t * head_dim.  One kernel (and a clear of
+ * v_norm_all) writes the summaries of the geom->max_blocks = ceil(length / block_size) blocks and
+ * everything in `extras`.  The means are summed per quarter of a block and
+ * the quarters pairwise; ia_build_summaries sums in token order: k_bar may differ in the last bit. */
+int ia_build_prompt_blocks(const void* k, const void* v, int length, const ia_geom* geom,
+                           const ia_summaries* summaries, const ia_prompt_extras* extras, ia_stream_t stream);
 
 /* Replaces the selection stats kernel plus the routing decision
  * (IMPL/core.py:751-814, IMPL/page_attention.py:84-171): condition score of

@@ -45,6 +45,13 @@ class Summaries(Structure):
                 ("v_norm_max", c_void_p), ("w", c_void_p), ("rho", c_void_p)]
 
 
+class PromptExtras(Structure):
+    _fields_ = [("v_bar_f32", c_void_p), ("k_max_f32", c_void_p), ("k_min_f32", c_void_p), ("k_block", c_void_p),
+                ("v_block", c_void_p), ("token_idx", c_void_p), ("valid_token", c_void_p), ("counts", c_void_p),
+                ("v_norm_all", c_void_p), ("table", c_void_p), ("prefix_len", c_void_p), ("seq_len", c_void_p),
+                ("table_entries", c_int32), ("reserved", c_int32)]
+
+
 class SelectAux(Structure):
     _fields_ = [("score", c_void_p), ("z", c_void_p), ("s", c_void_p), ("delta", c_void_p),
                 ("globals", c_void_p)]
@@ -72,6 +79,8 @@ SIGNATURES = {
     "ia_build_summaries": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, POINTER(Geom), POINTER(Summaries), c_void_p]),
     "ia_update_summaries": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, POINTER(Geom), POINTER(Summaries),
                                     c_void_p]),
+    "ia_build_prompt_blocks": (c_int, [c_void_p, c_void_p, c_int, POINTER(Geom), POINTER(Summaries),
+                                       POINTER(PromptExtras), c_void_p]),
     "ia_select": (c_int, [c_void_p, POINTER(Summaries), c_void_p, POINTER(Geom), c_int, c_int, c_float, c_int,
                           c_void_p, c_void_p, POINTER(SelectAux), c_void_p]),
     "ia_select_split": (c_int, [c_void_p, POINTER(Summaries), c_void_p, POINTER(Geom), c_int, c_int, c_int, c_int,

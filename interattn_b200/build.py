@@ -21,7 +21,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB_PATH = os.path.join(HERE, "libinterattn_b200.so")
-SOURCES = ["capi.cu", "summaries.cu", "select.cu", "select_inst_bf16_d128_range.cu", "select_inst_bf16_d128_diag.cu",
+SOURCES = ["capi.cu", "summaries.cu", "prompt_blocks.cu", "select.cu", "select_inst_bf16_d128_range.cu", "select_inst_bf16_d128_diag.cu",
            "select_inst_bf16_d64.cu", "select_inst_f32_d128.cu", "select_inst_f32_d64.cu",
            "select_inst_kbar16_d128.cu", "select_inst_kbar16_d64.cu", "select_inst_bf16_d128_packed.cu",
            "select_inst_bf16_d64_packed.cu", "select_inst_f32_packed.cu", "select_inst_kbar16_packed.cu", "sparse_decode.cu", "sparse_decode_mma.cu",

@@ -187,6 +187,26 @@ int ia_update_summaries(const void* k_pool, const void* v_pool, const int32_t* b
                                 (cudaStream_t)stream);
 }
 
+int ia_build_prompt_blocks(const void* k, const void* v, int length, const ia_geom* geom,
+                           const ia_summaries* summaries, const ia_prompt_extras* x, ia_stream_t stream) {
+  if (int s = check_geom(geom)) return s;
+  if (int s = check_summaries(summaries, geom, true)) return s;
+  if (!k || !v || !x) return fail(IA_ERR_BAD_ARG, "prompt_blocks: null argument");
+  if (geom->batch != 1 || length <= 0) return fail(IA_ERR_BAD_ARG, "prompt_blocks: batch %d, length %d", geom->batch, length);
+  if (geom->max_blocks != (int)ceil_div64(length, geom->block_size))
+    return fail(IA_ERR_BAD_ARG, "prompt_blocks: max_blocks %d for %d tokens", geom->max_blocks, length);
+  if ((geom->reserved & IA_GEOM_DIAG_ELL) || summaries->w || summaries->rho)
+    return fail(IA_ERR_UNSUPPORTED, "prompt_blocks: the diagonal-ellipsoid pair is not built here");
+  if (!aligned16(k) || !aligned16(v) || !aligned16(x->k_block) || !aligned16(x->v_block))
+    return fail(IA_ERR_BAD_ARG, "prompt_blocks: the caches and their copies must be 16-byte aligned");
+  if ((x->k_block == nullptr) != (x->v_block == nullptr) || x->reserved != 0 || x->table_entries < 0)
+    return fail(IA_ERR_BAD_ARG, "prompt_blocks: extras");
+  if (!x->v_norm_all || !x->prefix_len || !x->seq_len || (x->table_entries > 0 && !x->table) ||
+      !x->token_idx || !x->valid_token || !x->counts)
+    return fail(IA_ERR_BAD_ARG, "prompt_blocks: null member in extras");
+  return launch_prompt_blocks(k, v, length, *geom, *summaries, *x, (cudaStream_t)stream);
+}
+
 int ia_select(const void* q, const ia_summaries* summaries, const int32_t* prefix_lens,
               const ia_geom* geom, int mode, int top_k, float eps, int max_sel, int32_t* sel_idx,
               int32_t* sel_count, const ia_select_aux* aux, ia_stream_t stream) {

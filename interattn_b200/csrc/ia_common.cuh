@@ -158,6 +158,8 @@ constexpr float kLn2 = 0.6931471805599453f;
 int launch_build_summaries(const void* k_pool, const void* v_pool, const int32_t* block_table,
                            const int32_t* prefix_lens, const int32_t* first_blocks, const ia_geom& g,
                            const ia_summaries& out, cudaStream_t stream);
+int launch_prompt_blocks(const void* k, const void* v, int length, const ia_geom& g, const ia_summaries& s,
+                         const ia_prompt_extras& x, cudaStream_t stream);
 // split_counters (may be null): one int per (sequence, kv head), cleared by the selection
 // kernel for the attention kernel's fused finalize
 // exchange (may be null) + block range: split-KV across GPUs, this rank scores blocks [block_lo, block_hi)

@@ -60,12 +60,12 @@ class _CacheGeometry:
     identity block table.  Holds the small device tensors that description needs."""
 
     def __init__(self, device, max_tokens: int):
+        """Storage only: ``ia_build_prompt_blocks`` writes the table and the lengths."""
         self.device = device
-        self.capacity_pages = 0
-        self.table = None
-        self.prefix_lens = torch.zeros((1,), dtype=torch.int32, device=device)
-        self.seq_lens = torch.zeros((1,), dtype=torch.int32, device=device)
-        self.ensure(max_tokens)
+        self.capacity_pages = max((int(max_tokens) + PAGE - 1) // PAGE, 64)
+        self.table = torch.empty((1, self.capacity_pages), dtype=torch.int32, device=device)
+        self.prefix_lens = torch.empty((1,), dtype=torch.int32, device=device)
+        self.seq_lens = torch.empty((1,), dtype=torch.int32, device=device)
 
     def ensure(self, max_tokens: int) -> None:
         need = (int(max_tokens) + PAGE - 1) // PAGE
@@ -121,11 +121,8 @@ def _build_prompt_blocks(k_all: torch.Tensor, v_all: torch.Tensor, block_size: i
         raise ValueError(f"block_size {block_size} must be a multiple of {PAGE}, at most 128")
     lib = _lib.load()
     hkv, length, d = (int(x) for x in k_all.shape)
-    nb = max(1, (length + block_size - 1) // block_size)
+    nb = (length + block_size - 1) // block_size
     dev = k_all.device
-    geometry = _CacheGeometry(dev, length)
-    geometry.prefix_lens.fill_(length)
-    geometry.seq_lens.fill_(length)
     # the reference's switch for the storage of k_bar (core.py:428-446): bf16 only next to bf16 K/V
     k_bar_name = os.environ.get("CONDITION_BLOCK_K_BAR_DTYPE", "float32")
     if k_bar_name not in ("float32", "bfloat16"):
@@ -134,45 +131,57 @@ def _build_prompt_blocks(k_all: torch.Tensor, v_all: torch.Tensor, block_size: i
         raise ValueError("CONDITION_BLOCK_K_BAR_DTYPE=bfloat16 needs bfloat16 keys and values.")
     # the reference's switch for the packed coordinate range (core.py:490-499)
     packed = os.environ.get("CONDITION_BLOCK_TMA_BOUNDS") == "1"
-    summ = ops.BlockSummaries.empty(1, hkv, nb, d, k_all.dtype, dev, block_size, getattr(torch, k_bar_name),
-                                    packed_bounds=packed)
+    mixed = os.environ.get("CONDITION_BLOCK_MIXED_SUMMARIES") == "1"
+    pad = nb * block_size - length
+    # A copy that autograd should follow (the cache is part of a graph) is made by torch, below.
+    own_copy = pad > 0 and not (torch.is_grad_enabled() and (k_all.requires_grad or v_all.requires_grad))
+    copies = 0 if mixed or k_all.dtype == torch.float32 else 1 if packed else 3   # fp32 copies: v_bar, k_max, k_min
+
+    # One launch writes all of it (an empty prompt is refused there).
+    new, slab = k_all.new_empty, (1, hkv, nb, d)
+    k_bar = new(slab, dtype=getattr(torch, k_bar_name))
+    v_bar, k_max, k_min = new((3, *slab)).unbind(0)
+    v_norm_max, v_norm_all = new((1, hkv, nb), dtype=torch.float32), new((hkv,), dtype=torch.float32)
+    token_idx, counts = new((nb, block_size), dtype=torch.int64), new((nb,), dtype=torch.int64)
+    valid_token = new((nb, block_size), dtype=torch.bool)
+    f32 = new((copies, hkv, nb, d), dtype=torch.float32).unbind(0) if copies else ()
+    blocks = new((2, hkv, nb, block_size, d)).unbind(0) if own_copy else ()
+    k_bounds = None
+    if packed:   # the space of the two bound arrays as one array of pairs
+        k_bounds = k_max.as_strided((1, hkv, nb, 2 * d), (hkv * nb * 2 * d, nb * 2 * d, 2 * d, 1))
+        pairs = k_bounds.view(1, hkv, nb, d, 2)
+        k_max, k_min = pairs[..., 0], pairs[..., 1]
+    summ = ops.BlockSummaries(k_bar=k_bar, k_max=k_max, k_min=k_min, v_bar=v_bar, v_norm_max=v_norm_max,
+                              block_size=block_size, k_bounds=k_bounds)
+    geometry = _CacheGeometry(dev, length)
     g = geometry.geom(k_all, 1, block_size, nb, summ)
     s = summ.c_struct()
-    check(lib.ia_build_summaries(ctypes.c_void_p(k_all.data_ptr()), ctypes.c_void_p(v_all.data_ptr()),
-                                 ctypes.c_void_p(geometry.table.data_ptr()),
-                                 ctypes.c_void_p(geometry.prefix_lens.data_ptr()),
-                                 ctypes.byref(g), ctypes.byref(s), _stream()))
-    n_real = (length + block_size - 1) // block_size
-    token_idx = torch.arange(n_real * block_size, device=dev).reshape(n_real, block_size)
-    valid_token = token_idx < length
-    counts = valid_token.sum(dim=1).long()
-    mixed = os.environ.get("CONDITION_BLOCK_MIXED_SUMMARIES") == "1"
+    ptrs = [t.data_ptr() for t in f32] + [None] * (3 - len(f32)) + ([t.data_ptr() for t in blocks] or [None, None])
+    extras = _lib.PromptExtras(*ptrs, token_idx.data_ptr(), valid_token.data_ptr(), counts.data_ptr(),
+                               v_norm_all.data_ptr(), geometry.table.data_ptr(), geometry.prefix_lens.data_ptr(),
+                               geometry.seq_lens.data_ptr(), geometry.capacity_pages, 0)
+    check(lib.ia_build_prompt_blocks(ctypes.c_void_p(k_all.data_ptr()), ctypes.c_void_p(v_all.data_ptr()), length,
+                                     ctypes.byref(g), ctypes.byref(s), ctypes.byref(extras), _stream()))
 
-    def stored(t):
-        t = t[0, :, :n_real]
-        return t if mixed else t.float()
-
-    def blocked(x):
-        pad = n_real * block_size - length
+    def blocked(x, i):
+        if own_copy:
+            return blocks[i]
         if pad:
             x = torch.cat([x, x.new_zeros((hkv, pad, d))], dim=1)
-        return x.reshape(hkv, n_real, block_size, d)
+        return x.reshape(hkv, nb, block_size, d)
 
-    v_norm_max = summ.v_norm_max[0, :, :n_real]
     prefix = {
-        "k_block_attn": blocked(k_all), "v_block_attn": blocked(v_all),
+        "k_block_attn": blocked(k_all, 0), "v_block_attn": blocked(v_all, 1),
         "token_idx": token_idx, "valid_token": valid_token,
-        "k_bar": summ.k_bar[0, :, :n_real], "v_bar": stored(summ.v_bar),
-        "k_max": stored(summ.k_max), "k_min": stored(summ.k_min),
-        "v_norm_max": v_norm_max,
-        "v_norm_all": v_norm_max.amax(dim=-1) if n_real else v_norm_max.new_zeros((hkv,)),
+        "k_bar": k_bar[0], "v_bar": f32[0] if copies else v_bar[0],
+        "k_max": f32[1] if copies == 3 else k_max[0], "k_min": f32[2] if copies == 3 else k_min[0],
+        "v_norm_max": v_norm_max[0],
+        "v_norm_all": v_norm_all,
         "block_valid_counts": counts,
         "_b200": _PrefixHandle(k_all, v_all, block_size, summ, geometry),
     }
-    if packed:  # as the reference: the packed array, and k_max / k_min as views into it (no duplicate storage)
-        prefix["k_bounds"] = summ.k_bounds[0, :, :n_real]
-        pairs = prefix["k_bounds"].view(hkv, n_real, d, 2)
-        prefix["k_max"], prefix["k_min"] = pairs[..., 0], pairs[..., 1]
+    if packed:  # as the reference: the packed array next to the views into it (no duplicate storage)
+        prefix["k_bounds"] = k_bounds[0]
     return prefix
 
 

@@ -75,6 +75,59 @@ def test_build_prompt_blocks_keys_values_and_strided_view():
         assert torch.equal(prefix[key], dense[key])
 
 
+@pytest.mark.parametrize("mode", ["plain", "mixed", "packed", "kbar16"])
+@pytest.mark.parametrize("dtype,d,block", [(torch.bfloat16, 128, 64), (torch.bfloat16, 64, 48), (torch.float32, 128, 16),
+                                           (torch.float32, 64, 128)])
+@pytest.mark.parametrize("length", [1, 16, 63, 129, 1040, 3000])
+def test_build_prompt_blocks_edges(length, dtype, d, block, mode, monkeypatch):
+    """Every key of the prefix at the edges of tokens, pages and blocks, against torch on the same cache (NaN behind
+    the prompt's end must not show).  Means: at most 128 fp32 additions of N(0, 1) values and one division,
+    |error| < 1e-5; stored values and bounds are exact after their rounding; norms: one fp32 sum of squares."""
+    api = _api()
+    if mode == "kbar16" and dtype != torch.bfloat16:
+        pytest.skip("bf16 k_bar goes with bf16 caches")
+    for name, on in (("CONDITION_BLOCK_MIXED_SUMMARIES", mode == "mixed"), ("CONDITION_BLOCK_TMA_BOUNDS", mode == "packed")):
+        monkeypatch.setenv(name, "1" if on else "0")
+    monkeypatch.setenv("CONDITION_BLOCK_K_BAR_DTYPE", "bfloat16" if mode == "kbar16" else "float32")
+    hkv, spare = 3, 24
+    k, v = (x.to(DEV) for x in _cache(hkv, length, d, dtype, 40 + length, spare))
+    k[:, length:], v[:, length:] = float("nan"), float("nan")
+    p = api._build_prompt_blocks(k[:, :length], v[:, :length], block)
+    torch.cuda.synchronize()
+    nb = (length + block - 1) // block
+    pad = nb * block - length
+    idx = torch.arange(nb * block, device=DEV).reshape(nb, block)
+    assert torch.equal(p["token_idx"], idx) and torch.equal(p["valid_token"], idx < length)
+    assert torch.equal(p["block_valid_counts"], (idx < length).sum(dim=1))
+    kb, vb = (torch.cat([x[:, :length], x.new_zeros((hkv, pad, d))], dim=1).reshape(hkv, nb, block, d) for x in (k, v))
+    assert torch.equal(p["k_block_attn"], kb) and torch.equal(p["v_block_attn"], vb)
+    dead = (idx >= length)[None, :, :, None]
+    stored = dtype if mode in ("mixed",) else torch.float32
+    hi, lo = (kb.float().masked_fill(dead, s * float("inf")) for s in (-1.0, 1.0))
+    for name, want in (("k_max", hi.amax(dim=2)), ("k_min", lo.amin(dim=2))):
+        assert p[name].dtype == (dtype if mode == "packed" else stored) and torch.equal(p[name].float(), want)
+    if mode == "packed":
+        assert p["k_bounds"].shape == (hkv, nb, 2 * d)
+        assert torch.equal(p["k_bounds"].view(hkv, nb, d, 2)[..., 0], p["k_max"])
+    counts = (idx < length).sum(dim=1)[None, :, None]
+    for name, x in (("k_bar", kb), ("v_bar", vb)):
+        want = x.double().sum(dim=2) / counts
+        got = p[name].double()
+        rounded = dtype == torch.bfloat16 and (name == "v_bar" or mode == "kbar16")
+        torch.testing.assert_close(got, want, rtol=2 ** -8 if rounded else 0, atol=1e-5)
+        assert p[name].dtype == ((torch.bfloat16 if mode == "kbar16" else torch.float32) if name == "k_bar" else stored)
+        if rounded:   # the copy holds the stored value
+            assert torch.equal(got, got.to(torch.bfloat16).double())
+    norm = (vb.double() ** 2).sum(dim=3).amax(dim=2).sqrt()
+    torch.testing.assert_close(p["v_norm_max"].double(), norm, rtol=2e-6, atol=0)
+    assert torch.equal(p["v_norm_all"], p["v_norm_max"].amax(dim=-1))
+    with pytest.raises(ValueError):
+        api._build_prompt_blocks(k[:, :0], v[:, :0], block)
+    geo = p["_b200"].geometry
+    assert torch.equal(geo.table.view(-1), torch.arange(geo.capacity_pages, device=DEV, dtype=torch.int32))
+    assert geo.prefix_lens.tolist() == [length] and geo.seq_lens.tolist() == [length]
+
+
 def test_select_and_stats_shims():
     api = _api()
     hkv, g, d, block, length = 4, 4, 128, 64, 1500
