@@ -379,7 +379,9 @@ int ia_suggest_splits(const ia_geom* geom, int expected_blocks) {
   int best = 1;
   double best_t = 1e30;
   for (int s = 1; s <= 16; ++s) {
-    if (s > 1 && pages / s < 8) break;  // keep at least two pages per warp
+    // keep at least two pages per warp; the fp32 kernel takes a page in one round trip and is called for little
+    // work: one page per warp (4 pairs x 16 pages: 4 parts instead of 2)
+    if (s > 1 && pages / s < (geom->dtype == IA_F32 ? 4 : 8)) break;
     const double cta_bytes = pair_bytes / s;
     double left = pairs * s, t = 0.0;
     while (left > 0.0) {
