@@ -85,7 +85,8 @@ typedef struct ia_geom {
   int32_t max_pages;    /* row length of block_table */
   int32_t max_blocks;   /* blocks per (sequence, kv head) in the summary arrays */
   int32_t dtype;        /* ia_dtype of q, pools, k_max/k_min/v_bar */
-  int32_t reserved;     /* flags: IA_GEOM_KBAR_BF16 | IA_GEOM_DIAG_ELL | IA_GEOM_PACKED_BOUNDS, else 0 */
+  int32_t reserved;     /* flags: IA_GEOM_KBAR_BF16 | IA_GEOM_DIAG_ELL | IA_GEOM_PACKED_BOUNDS |
+                           IA_GEOM_SUFFIX_LENS, else 0 */
   int32_t n_pool_pages; /* physical pages in k_pool / v_pool; block-table entries are checked against
                            it before they are used.  0: unknown, entries are trusted. */
   int32_t reserved2;    /* 0 */
@@ -113,6 +114,9 @@ typedef struct ia_geom {
  * writes that layout, ia_select / ia_decode_attention read it (same bytes per block as the two arrays).
  * Not together with IA_GEOM_DIAG_ELL. */
 #define IA_GEOM_PACKED_BOUNDS 4
+/* ia_geom.reserved flag: the seq_lens argument of the decode calls holds the length of the generated suffix
+ * alone (the reference's suffix_len_dev, IMPL/core.py:1238-1244); a sequence is prefix + suffix long. */
+#define IA_GEOM_SUFFIX_LENS 8
 
 /* Block summaries, "mixed" storage of the reference (IMPL/core.py:411-446):
  * means accumulated in fp32, k_bar kept in fp32, the rest in the KV dtype

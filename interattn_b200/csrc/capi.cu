@@ -65,7 +65,7 @@ int check_geom(const ia_geom* g) {
   const int64_t esz = g->dtype == IA_BF16 ? 2 : 4;
   if ((g->pool_head_stride * esz) % 16 != 0 || (g->pool_page_stride * esz) % 16 != 0)
     return fail(IA_ERR_BAD_ARG, "geom: pool strides must be multiples of 16 bytes");
-  if (g->reserved & ~(IA_GEOM_KBAR_BF16 | IA_GEOM_DIAG_ELL | IA_GEOM_PACKED_BOUNDS))
+  if (g->reserved & ~(IA_GEOM_KBAR_BF16 | IA_GEOM_DIAG_ELL | IA_GEOM_PACKED_BOUNDS | IA_GEOM_SUFFIX_LENS))
     return fail(IA_ERR_BAD_ARG, "geom: unknown flag bits in reserved (%d)", g->reserved);
   if ((g->reserved & IA_GEOM_DIAG_ELL) && (g->reserved & IA_GEOM_PACKED_BOUNDS))
     return fail(IA_ERR_BAD_ARG, "geom: the packed range layout and the diag_ell bound exclude one another");

@@ -21,6 +21,7 @@ struct DecodeParams {
   const int32_t* block_table;
   const int32_t* prefix_lens;
   const int32_t* seq_lens;
+  int suffix_lens;  // seq_lens holds suffix lengths (IA_GEOM_SUFFIX_LENS)
   const int32_t* sel_idx;
   const int32_t* sel_count;
   const void* v_bar;  // hybrid only
@@ -104,7 +105,7 @@ __device__ __forceinline__ ItemRange item_range(const DecodeParams& p, int seq, 
   // lengths come from device memory: never index the block table past its row
   const int capacity = p.max_pages * p.page_size;
   r.prefix = min(max(p.prefix_lens[seq], 0), capacity);
-  r.seq_len = min(p.seq_lens[seq], capacity);
+  r.seq_len = min(p.seq_lens[seq] + (p.suffix_lens ? p.prefix_lens[seq] : 0), capacity);
   r.nb_eff = min((r.prefix + p.block_size - 1) / p.block_size, p.max_blocks);
   r.lo_b = max(p.block_lo, 0);
   r.hi_b = min(p.block_hi, r.nb_eff);
@@ -247,7 +248,7 @@ __device__ __forceinline__ PairItems pair_items(const DecodeParams& p, int pair)
   const int seq = pair / p.n_kv_heads;
   const int capacity = p.max_pages * p.page_size;
   r.prefix = min(max(p.prefix_lens[seq], 0), capacity);
-  r.seq_len = min(p.seq_lens[seq], capacity);
+  r.seq_len = min(p.seq_lens[seq] + (p.suffix_lens ? p.prefix_lens[seq] : 0), capacity);
   r.nb_eff = min((r.prefix + p.block_size - 1) / p.block_size, p.max_blocks);
   const int count = max(min(p.sel_count[pair], p.max_sel), 0);
   r.n_sel_items = count * (p.block_size / p.page_size);

@@ -78,6 +78,7 @@ struct SelectParams {
     int heads_outer;      // the pools' tensor maps are [kv head, page, token, head_dim] (head stride > page stride)
     const int32_t* block_table;
     const int32_t* seq_lens;
+    int suffix_lens;  // seq_lens holds suffix lengths (IA_GEOM_SUFFIX_LENS)
     void* out;
     int max_pages, n_pool_pages;
     int ring_bytes;  // shared memory of the ring (the selection's stages), reused for the pages
@@ -536,7 +537,7 @@ __device__ __forceinline__ void attend_selected_pages(const SelectParams& p, int
   const int ppb = p.block_size / kPage;
   const int cap = p.att.max_pages * kPage;
   const int prefix = min(prefix_raw, cap);
-  const int seq_len = min(max(p.att.seq_lens[seq], prefix), cap);
+  const int seq_len = min(max(p.att.seq_lens[seq] + (p.att.suffix_lens ? prefix_raw : 0), prefix), cap);
   const int n_sel_items = count * ppb;
   const int suf_first = prefix / kPage;
   const int n_suf = seq_len > prefix ? (seq_len - 1) / kPage - suf_first + 1 : 0;
@@ -2060,6 +2061,7 @@ static bool try_launch_fused(SelectParams& p, const AttendRequest& ar, int n_pai
     }
     p.att.block_table = ar.req->block_table;
     p.att.seq_lens = ar.req->seq_lens;
+    p.att.suffix_lens = (g.reserved & IA_GEOM_SUFFIX_LENS) != 0;
     p.att.out = ar.req->out;
     p.att.max_pages = g.max_pages;
     p.att.n_pool_pages = g.n_pool_pages;

@@ -276,7 +276,7 @@ int launch_sparse_decode(const void* q, const void* k_pool, const void* v_pool,
   p.trace = getenv("IA_TRACE_PTR") ? reinterpret_cast<float*>(strtoull(getenv("IA_TRACE_PTR"), nullptr, 16)) : nullptr;
 #endif
   p.q = q; p.k_pool = k_pool; p.v_pool = v_pool; p.block_table = block_table;
-  p.prefix_lens = prefix_lens; p.seq_lens = seq_lens; p.sel_idx = sel_idx; p.sel_count = sel_count;
+  p.prefix_lens = prefix_lens; p.seq_lens = seq_lens; p.suffix_lens = (g.reserved & IA_GEOM_SUFFIX_LENS) != 0; p.sel_idx = sel_idx; p.sel_count = sel_count;
   p.v_bar = summaries ? summaries->v_bar : nullptr;
   p.z = z;
   p.o_partial = o_partial; p.lse_partial = lse_partial;

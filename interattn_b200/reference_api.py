@@ -94,6 +94,9 @@ class _PrefixHandle:
         self.prompt_len = int(k_all.shape[1])
         self.summ = summ
         self.geometry = geometry
+        # the decode step is called once per layer and token: its constant arguments in the form the library takes
+        self.c_summ = summ.c_struct()
+        self.geom_flags = ops._geom_flags(summ) | _lib.IA_GEOM_SUFFIX_LENS
 
 
 def _stream():
@@ -262,10 +265,10 @@ def _run_condition_block_selection_stats(q_grouped, prefix, workspace=None, redu
 
 class _StepWorkspace:
     """Device scratch of one layer, reused across steps (the reference keeps a
-    dict of tensors per layer; this object lives in that dict)."""
+    dict of tensors per layer; this object lives in that dict), and the geometry struct it was sized for."""
 
-    def __init__(self, lib, geom: Geom, max_sel: int, n_splits: int, rep_mode: int, device, dtype, rows, d):
-        self.key = (geom.n_kv_heads, geom.group_size, geom.max_blocks, max_sel, n_splits, rep_mode, dtype)
+    def __init__(self, lib, geom: Geom, key, max_sel: int, n_splits: int, rep_mode: int, device, dtype, rows, d):
+        self.key, self.geom = key, geom
         need = lib.ia_workspace_bytes(ctypes.byref(geom), max_sel, n_splits, rep_mode)
         if need < 0:
             check(_lib.IA_ERR_BAD_ARG)
@@ -276,19 +279,18 @@ class _StepWorkspace:
         self.sel_count = torch.empty((1, geom.n_kv_heads), device=device, dtype=torch.int32)
         self.out = torch.empty((1, rows, d), device=device, dtype=dtype)
 
-    def ptr(self):
-        return ctypes.c_void_p(self.buf.data_ptr() + self.off)
-
 
 def _suffix_continues_prefix(h: _PrefixHandle, k_suffix, v_suffix) -> bool:
-    esz = h.k_all.element_size()
-    d = int(h.k_all.shape[2])
+    """Does the suffix lie right behind the prefix, in the same storage and with the same strides?"""
     for cache, suf in ((h.k_all, k_suffix), (h.v_all, v_suffix)):
-        if suf.dim() != 3 or suf.dtype != cache.dtype or suf.shape[0] != cache.shape[0] or suf.shape[2] != d:
+        hkv, length, d = cache.shape
+        if suf.dim() != 3 or suf.dtype != cache.dtype:
             return False
-        if suf.shape[1] and (suf.stride(2) != 1 or suf.stride(1) != d or suf.stride(0) != cache.stride(0)):
+        s_hkv, n, s_d = suf.shape
+        if s_hkv != hkv or s_d != d:
             return False
-        if suf.shape[1] and suf.data_ptr() != cache.data_ptr() + h.prompt_len * d * esz:
+        if n and (suf.stride() != (cache.stride(0), d, 1)
+                  or suf.data_ptr() != cache.data_ptr() + length * d * cache.element_size()):
             return False
     return True
 
@@ -305,61 +307,75 @@ def _condition_block_decode_output_fused_triton(
     then read prefix and suffix in place.  ``kv_cache=(k_all, v_all)`` names the
     current full cache explicitly (a dynamic cache is re-allocated every step).
     Any other suffix tensor is supported through a slow path that copies prefix
-    and suffix into one contiguous cache first."""
+    and suffix into one contiguous cache first.
+
+    This is the reference's per layer and token call, and the host bounds it: what does not change from
+    call to call (structs, sizes) lives in the handle and the workspace, the suffix length is read by the kernels
+    where it lies, and pointers go to the library as plain integers.  One sequence, 8192 tokens, epsilon rule:
+    38.6 -> 23.8 us per call in a queue of calls, 22.6 of them the kernel."""
     if rep_mode not in _REP:
         raise ValueError(f"rep_mode must be one of {sorted(_REP)}")
     lib = _lib.load()
     h = _handle(prompt_prefix)
     if int(page_size) != h.block_size:
         raise ValueError(f"page_size {page_size} differs from the block size {h.block_size} of the prefix")
-    hkv, d = int(h.k_all.shape[0]), int(h.k_all.shape[2])
-    group, q = _check_q(q_grouped.to(h.k_all.dtype), hkv, d)
-    nb = h.summ.max_blocks
-    n_real = int(prompt_prefix["block_valid_counts"].numel())
+    cache = h.k_all
+    hkv, prompt_len, d = cache.shape
+    dtype = cache.dtype
+    if q_grouped.dim() != 4 or q_grouped.shape[0] != hkv or q_grouped.shape[3] != d:
+        raise ValueError("q_grouped must be [Hkv, G, 1, D]")
+    group = q_grouped.shape[1]
+    if q_grouped.shape[2] != 1:
+        raise ValueError("Triton selection stats expects q_len=1.")
+    q = q_grouped.to(dtype).contiguous()
+    n_suffix = k_suffix.shape[1]
     if kv_cache is not None:
         k_all, v_all = kv_cache
         _check_cache_view(k_all, "kv_cache[0]")
         _check_cache_view(v_all, "kv_cache[1]")
     elif _suffix_continues_prefix(h, k_suffix, v_suffix):
-        k_all, v_all = h.k_all, h.v_all      # base pointers; the suffix follows in the same storage
+        k_all, v_all = cache, h.v_all        # base pointers; the suffix follows in the same storage
     else:                                    # slow path: materialise one cache
-        k_all = torch.cat([h.k_all, k_suffix.to(h.k_all.dtype)], dim=1).contiguous()
-        v_all = torch.cat([h.v_all, v_suffix.to(h.v_all.dtype)], dim=1).contiguous()
+        k_all = torch.cat([cache, k_suffix.to(dtype)], dim=1).contiguous()
+        v_all = torch.cat([h.v_all, v_suffix.to(dtype)], dim=1).contiguous()
     geo = h.geometry
-    geo.ensure(h.prompt_len + int(k_suffix.shape[1]) + 1)
+    geo.ensure(prompt_len + n_suffix + 1)
     if not (torch.is_tensor(suffix_len_dev) and suffix_len_dev.is_cuda):
         raise ValueError("suffix_len_dev must be a CUDA int32 scalar tensor")
-    torch.add(geo.prefix_lens, suffix_len_dev.reshape(1).to(torch.int32), out=geo.seq_lens)
+    if suffix_len_dev.dtype != torch.int32 or suffix_len_dev.numel() != 1:
+        suffix_len_dev = suffix_len_dev.reshape(1).to(torch.int32)
 
     mode = IA_SELECT_TOPK if top_k is not None else IA_SELECT_EPS
     if term1_mass_exp:
         mode |= _lib.IA_SELECT_TERM1_MASS_EXP
-    max_sel = max(nb, 1)
-    g = geo.geom(k_all, group, h.block_size, nb, h.summ,
-                 n_tokens=max(int(k_all.shape[1]), h.prompt_len + int(k_suffix.shape[1])))
+    nb = h.summ.max_blocks
+    rep = _REP[rep_mode]
     ws_dict = workspace if workspace is not None else {}
-    n_splits = ws_dict.get("b200_n_splits")
-    if n_splits is None:
-        expect = min(int(top_k), nb) if top_k is not None else max(1, nb // 16)
-        n_splits = int(lib.ia_suggest_splits(ctypes.byref(g), expect))
-        ws_dict["b200_n_splits"] = n_splits
     ws = ws_dict.get("b200_step")
-    key = (hkv, group, nb, max_sel, n_splits, _REP[rep_mode], k_all.dtype)
+    n_splits = ws_dict.get("b200_n_splits")
+    n_tokens = max(k_all.shape[1], prompt_len + n_suffix)
+    key = (hkv, group, nb, n_splits, rep, k_all.dtype, d)
     if ws is None or ws.key != key or ws.buf.device != q.device:
-        ws = _StepWorkspace(lib, g, max_sel, n_splits, _REP[rep_mode], q.device, k_all.dtype, hkv * group, d)
+        g = geo.geom(k_all, group, h.block_size, nb, h.summ)
+        if n_splits is None:
+            expect = min(int(top_k), nb) if top_k is not None else max(1, nb // 16)
+            n_splits = int(lib.ia_suggest_splits(ctypes.byref(g), expect))
+            ws_dict["b200_n_splits"] = n_splits
+            key = (hkv, group, nb, n_splits, rep, k_all.dtype, d)
+        ws = _StepWorkspace(lib, g, key, nb, n_splits, rep, q.device, k_all.dtype, hkv * group, d)
         ws_dict["b200_step"] = ws
-    s = h.summ.c_struct()
+    g = ws.geom                              # what the key does not fix
+    g.block_size, g.reserved = h.block_size, h.geom_flags
+    g.max_pages, g.n_pool_pages, g.pool_head_stride = geo.capacity_pages, (n_tokens + PAGE - 1) // PAGE, k_all.stride(0)
     check(lib.ia_decode_attention(
-        ctypes.c_void_p(q.data_ptr()), ctypes.c_void_p(k_all.data_ptr()), ctypes.c_void_p(v_all.data_ptr()),
-        ctypes.c_void_p(geo.table.data_ptr()), ctypes.c_void_p(geo.prefix_lens.data_ptr()),
-        ctypes.c_void_p(geo.seq_lens.data_ptr()), ctypes.byref(s), ctypes.byref(g), mode, int(top_k or 0),
-        float(eps or 0.0), max_sel, _REP[rep_mode], n_splits, ws.ptr(), ws.bytes,
-        ctypes.c_void_p(ws.sel_idx.data_ptr()), ctypes.c_void_p(ws.sel_count.data_ptr()),
-        ctypes.c_void_p(ws.out.data_ptr()), _stream()))
-    out = ws.out.reshape(hkv, group, 1, d)
+        q.data_ptr(), k_all.data_ptr(), v_all.data_ptr(), geo.table.data_ptr(), geo.prefix_lens.data_ptr(),
+        suffix_len_dev.data_ptr(), ctypes.byref(h.c_summ), ctypes.byref(g), mode, int(top_k or 0), float(eps or 0.0),
+        nb, rep, n_splits, ws.buf.data_ptr() + ws.off, ws.bytes, ws.sel_idx.data_ptr(), ws.sel_count.data_ptr(),
+        ws.out.data_ptr(), torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())))
+    out = ws.out.view(hkv, group, 1, d)
     if output_dtype is not None and out.dtype != output_dtype:
         out = out.to(output_dtype)
-    selected = _mask_from_indices(ws.sel_idx, n_real, group) if store_selected else None
+    selected = _mask_from_indices(ws.sel_idx, prompt_prefix["block_valid_counts"].numel(), group) if store_selected else None
     return out, selected
 
 

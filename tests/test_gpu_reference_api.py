@@ -236,6 +236,33 @@ def test_fused_decode_sanity_cases(prompt_len, suffix_len, eps, suffix_is_view):
     assert float(diff) < 2e-2
 
 
+@pytest.mark.parametrize("suffix_len", [0, 1, 33])
+@pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 128), (torch.bfloat16, 64), (torch.float32, 64), (torch.float32, 128)])
+def test_suffix_length_read_on_the_device(dtype, d, suffix_len):
+    """The kernels add the prefix to the suffix length themselves (one-kernel step, tensor-core and FMA attention):
+    the length may change on the device between two calls, int64 lengths are converted, and NaN behind the
+    sequence's end must not show.  fp32: sums of a few hundred terms; bf16: the output's rounding and P in bf16."""
+    api = _api()
+    hkv, g, block, prompt = 2, 4, 64, 333
+    k, v = _cache(hkv, prompt + 40, d, dtype, 77)
+    k[:, prompt + suffix_len:], v[:, prompt + suffix_len:] = float("nan"), float("nan")
+    kd, vd = k.to(DEV), v.to(DEV)
+    q = torch.randn((hkv, g, 1, d), generator=torch.Generator().manual_seed(5)).to(dtype)
+    prefix = api._build_prompt_blocks(kd[:, :prompt], vd[:, :prompt], block)
+    length, ws = torch.zeros((), dtype=torch.int32, device=DEV), {}
+    args = dict(q_grouped=q.to(DEV), prompt_prefix=prefix, k_suffix=kd[:, prompt:prompt + 40], v_suffix=vd[:, prompt:prompt + 40],
+                eps=None, top_k=3, page_size=block, store_selected=False, output_dtype=dtype, workspace=ws)
+    api._condition_block_decode_output_fused_triton(suffix_len_dev=length, **args)
+    length.fill_(suffix_len)
+    got = api._condition_block_decode_output_fused_triton(suffix_len_dev=length, **args)[0].clone()
+    again = api._condition_block_decode_output_fused_triton(suffix_len_dev=length.long().view(1), **args)[0].clone()
+    n = prompt + suffix_len
+    want, *_ = _oracle_step(q, k[:, :n], v[:, :n], prompt, block, top_k=3)
+    tol = dict(rtol=1e-4, atol=1e-5) if dtype == torch.float32 else dict(rtol=1e-2, atol=2e-2)
+    torch.testing.assert_close(got[:, :, 0].float().cpu(), want.float(), **tol)
+    assert torch.equal(got, again)
+
+
 def test_fused_decode_topk_and_workspace_reuse():
     api = _api()
     hkv, g, d, block, prompt_len = 2, 8, 128, 64, 2000
