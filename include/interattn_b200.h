@@ -488,6 +488,31 @@ int64_t ia_llama_gemm_workspace_bytes(int n);
 int ia_llama_gemm(const void* x, const void* w_packed, void* out, int m, int n, int k, void* workspace,
                   int64_t workspace_bytes, ia_stream_t stream);
 
+/* The same product over row-major weights with the sums left unfinished, for consumers that read it once - the
+ * form the fused decode step runs.  Every CTA writes its fp32 share of a tile of 128 output columns into a slot of
+ * `parts` (ia_llama_gemm_parts_bytes(n, k) bytes, 16-byte aligned, nothing to clear), and the ia_llama_*_parts call that
+ * follows on the stream - given the same parts and the k of the product - adds the slots in a fixed order, rounds to
+ * bf16 and goes on as its namesake above does on the finished projection.  x, w: 16-byte aligned, k a multiple of 8,
+ * m <= 16.  `out` (bf16 [m, n], else null): tiles that one CTA summed alone are written there instead, finished;
+ * ia_llama_argmax_parts completes the others.
+ *   add_rmsnorm_parts: n = hidden (a multiple of 8)
+ *   rope_append_parts: n = (n_q_heads + 2 n_kv_heads) * head_dim, head_dim a multiple of 8; tables, caches and q_out
+ *                      8-byte aligned
+ *   silu_mul_parts:    n = 2 * intermediate (intermediate a multiple of 8)
+ *   argmax_parts:      n = vocab; logits = the product's `out` */
+int64_t ia_llama_gemm_parts_bytes(int n, int k);
+int ia_llama_gemm_parts(const void* x, const void* w, void* out, int m, int n, int k, void* parts, int64_t parts_bytes,
+                        ia_stream_t stream);
+int ia_llama_add_rmsnorm_parts(void* residual, const void* parts, int k, const void* weight, void* out, int n_rows,
+                               int hidden, float eps, ia_stream_t stream);
+int ia_llama_rope_append_parts(const void* parts, int k, const void* cos_table, const void* sin_table, int max_pos,
+                               const int32_t* seq_lens, void* k_cache, void* v_cache, int64_t cache_seq_stride,
+                               int64_t cache_head_stride, int cache_len, void* q_out, int batch, int n_q_heads,
+                               int n_kv_heads, int head_dim, ia_stream_t stream);
+int ia_llama_silu_mul_parts(const void* parts, int k, void* out, int n_rows, int intermediate, ia_stream_t stream);
+int ia_llama_argmax_parts(const void* parts, int k, void* logits, int n_rows, int vocab, int64_t* out,
+                          ia_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

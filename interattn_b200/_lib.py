@@ -119,6 +119,14 @@ SIGNATURES = {
     "ia_llama_gemm_packed_bytes": (c_int64, [c_int, c_int]),
     "ia_llama_gemm_pack": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "ia_llama_gemm_workspace_bytes": (c_int64, [c_int]),
+    "ia_llama_gemm_parts_bytes": (c_int64, [c_int, c_int]),
+    "ia_llama_gemm_parts": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int64, c_void_p]),
+    "ia_llama_add_rmsnorm_parts": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_float,
+                                           c_void_p]),
+    "ia_llama_rope_append_parts": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
+                                           c_int64, c_int64, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
+    "ia_llama_silu_mul_parts": (c_int, [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p]),
+    "ia_llama_argmax_parts": (c_int, [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "ia_llama_gemm": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int64, c_void_p]),
 }
 

@@ -11,7 +11,7 @@
 // step agree to the last bit except for the order of the fp32 sum of squares.
 //
 // All tensors are bf16, rows are contiguous.
-#include "ia_common.cuh"
+#include "gemm_parts.cuh"
 
 namespace ia {
 namespace {
@@ -190,6 +190,227 @@ llama_argmax_kernel(const __nv_bfloat16* __restrict__ logits, int64_t row_stride
   }
 }
 
+// ---- the same kernels on a projection's partial sums (gemm_parts.cuh) ---------------------------------
+// Latency bound: a few hundred KB out of L2 and one row reduction.  The sums of a column's slots replace the load of
+// the finished projection (up to eight slots in flight at once); everything after that, rounding points included, is
+// the kernel above.
+constexpr int kPartNormThreads = 512;
+template <int kChunks>
+__global__ void __launch_bounds__(kPartNormThreads)
+llama_add_rmsnorm_parts_kernel(__nv_bfloat16* __restrict__ residual, const PartsView parts,
+                               const __nv_bfloat16* __restrict__ weight, __nv_bfloat16* __restrict__ out, int hidden,
+                               float eps) {
+  grid_launch_dependents();
+  float w[kChunks][8];  // weights do not depend on the kernel before
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) {
+    const int i = (c * kPartNormThreads + threadIdx.x) * 8;
+    if (i < hidden) load8(weight + i, w[c]);
+  }
+  grid_dependency_wait();
+  const int64_t row = (int64_t)blockIdx.x * hidden;
+  float x[kChunks][8];
+  float sq = 0.f;
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) {
+    const int i = (c * kPartNormThreads + threadIdx.x) * 8;
+    if (i < hidden) {
+      load8(residual + row + i, x[c]);
+      int count;
+      const float* tile = parts.tile((uint32_t)i / kPartCols, count);
+      float d[8];
+      sum_parts<8, 8>(tile, count, blockIdx.x, i % kPartCols, d);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[c][j] = round_bf16(x[c][j] + d[j]);
+      store8(residual + row + i, x[c]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sq = fmaf(x[c][j], x[c][j], sq);
+    }
+  }
+  __shared__ float part[kPartNormThreads / 32];
+  sq = warp_sum(sq);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sq;
+  __syncthreads();
+  float v = (threadIdx.x & 31) < kPartNormThreads / 32 ? part[threadIdx.x & 31] : 0.f;
+  const float scale = rsqrtf(warp_sum(v) / (float)hidden + eps);  // every warp for itself: the same order, one barrier
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) {
+    const int i = (c * kPartNormThreads + threadIdx.x) * 8;
+    if (i < hidden) {
+      float y[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) y[j] = w[c][j] * round_bf16(x[c][j] * scale);
+      store8(out + row + i, y);
+    }
+  }
+}
+
+__device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&v)[4]) {
+  const uint2 w = *reinterpret_cast<const uint2*>(p);
+  v[0] = bf16lo(w.x); v[1] = bf16hi(w.x); v[2] = bf16lo(w.y); v[3] = bf16hi(w.y);
+}
+__device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&v)[4]) {
+  uint2 w;
+  w.x = pack2(v[0], v[1]); w.y = pack2(v[2], v[3]);
+  *reinterpret_cast<uint2*>(p) = w;
+}
+
+// One thread per four coordinates of both halves of a head: unit = (sequence, head, d / 4)
+__global__ void __launch_bounds__(128)
+llama_rope_append_parts_kernel(const PartsView parts, const __nv_bfloat16* __restrict__ cos_t,
+                               const __nv_bfloat16* __restrict__ sin_t, int max_pos,
+                               const int32_t* __restrict__ seq_lens, __nv_bfloat16* __restrict__ k_cache,
+                               __nv_bfloat16* __restrict__ v_cache, int64_t seq_stride, int64_t head_stride,
+                               int cache_len, __nv_bfloat16* __restrict__ q_out, int batch, int n_q_heads,
+                               int n_kv_heads, int D) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int half = D >> 1, per_head = D >> 3, n_heads = n_q_heads + 2 * n_kv_heads;
+  const int unit = blockIdx.x * 128 + threadIdx.x;
+  if (unit >= batch * n_heads * per_head) return;
+  const int d = (unit % per_head) * 4, head = unit / per_head % n_heads, b = unit / (per_head * n_heads);
+  const int pos = seq_lens[b] - 1;
+  if (pos < 0 || pos >= max_pos || pos >= cache_len) return;
+  float x1[4], x2[4];
+  {
+    const int c1 = head * D + d, c2 = c1 + half;
+    int n1, n2;
+    const float* t1 = parts.tile((uint32_t)c1 / kPartCols, n1);
+    const float* t2 = parts.tile((uint32_t)c2 / kPartCols, n2);
+    sum_parts<4, 8>(t1, n1, b, c1 % kPartCols, x1);
+    sum_parts<4, 8>(t2, n2, b, c2 % kPartCols, x2);
+  }
+  if (head >= n_q_heads + n_kv_heads) {  // value head: plain copy
+    __nv_bfloat16* dst = v_cache + b * seq_stride + (head - n_q_heads - n_kv_heads) * head_stride + (int64_t)pos * D;
+    store4(dst + d, x1);
+    store4(dst + d + half, x2);
+    return;
+  }
+  float c1[4], c2[4], s1[4], s2[4], lo[4], hi[4];
+  load4(cos_t + (int64_t)pos * D + d, c1);
+  load4(cos_t + (int64_t)pos * D + d + half, c2);
+  load4(sin_t + (int64_t)pos * D + d, s1);
+  load4(sin_t + (int64_t)pos * D + d + half, s2);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    lo[j] = round_bf16(x1[j] * c1[j]) + round_bf16(-x2[j] * s1[j]);
+    hi[j] = round_bf16(x2[j] * c2[j]) + round_bf16(x1[j] * s2[j]);
+  }
+  __nv_bfloat16* dst = head < n_q_heads
+                           ? q_out + ((int64_t)b * n_q_heads + head) * D
+                           : k_cache + b * seq_stride + (head - n_q_heads) * head_stride + (int64_t)pos * D;
+  store4(dst + d, lo);
+  store4(dst + d + half, hi);
+}
+
+__global__ void __launch_bounds__(256)
+llama_silu_mul_parts_kernel(const PartsView parts, __nv_bfloat16* __restrict__ out, int n_rows, int inter) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int per_row = inter >> 3;
+  const int64_t unit = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (unit >= (int64_t)n_rows * per_row) return;
+  const int r = (int)(unit / per_row);
+  const int i = (int)(unit - (int64_t)r * per_row) * 8;
+  float g[8], u[8], y[8];
+  int ng, nu;
+  const float* tg = parts.tile((uint32_t)i / kPartCols, ng);
+  const float* tu = parts.tile((uint32_t)(inter + i) / kPartCols, nu);
+  sum_parts<8, 4>(tg, ng, r, i % kPartCols, g);
+  sum_parts<8, 4>(tu, nu, r, (inter + i) % kPartCols, u);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) y[j] = round_bf16(g[j] / (1.f + expf(-g[j]))) * u[j];
+  store8(out + (int64_t)r * inter + i, y);
+}
+
+// Completes the logits whose tiles several CTAs summed, then the arg-max.  A row is shared by a cluster of CTAs,
+// each with a run of whole tiles, and merged through rank 0's shared memory: a few rows alone would leave
+// most SMs idle (one CTA of 1024 threads per row takes 6.4 us at 128256 columns, this form ends 3 us after the product).
+constexpr int kArgmaxPartsThreads = 512, kArgmaxCluster = 8;
+__global__ void __cluster_dims__(kArgmaxCluster, 1, 1) __launch_bounds__(kArgmaxPartsThreads)
+llama_argmax_parts_kernel(const PartsView parts, __nv_bfloat16* __restrict__ logits, int vocab,
+                          int64_t* __restrict__ out) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  __shared__ float best_s[kArgmaxPartsThreads / 32];
+  __shared__ int idx_s[kArgmaxPartsThreads / 32];
+  __shared__ float rank_best[kArgmaxCluster];
+  __shared__ int rank_idx[kArgmaxCluster];
+  const int rank = blockIdx.x % kArgmaxCluster, row_i = blockIdx.x / kArgmaxCluster;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __nv_bfloat16* row = logits + (int64_t)row_i * vocab;
+  const int n_tiles = (vocab + kPartCols - 1) / kPartCols;
+  const int t_lo = (int)((int64_t)n_tiles * rank / kArgmaxCluster), t_hi = (int)((int64_t)n_tiles * (rank + 1) / kArgmaxCluster);
+  // A tile is split where a CTA's range starts inside it.  The boundaries T c / P are walked by the warps; the first
+  // boundary inside a tile stands for it.
+  const bool pairs = (vocab & 3) == 0;  // rows start on 8-byte boundaries
+  const uint32_t c_lo = max(parts.owner((uint32_t)t_lo * parts.k_chunks), 1u) ;
+  const uint32_t c_hi = t_hi > t_lo ? parts.owner((uint32_t)t_hi * parts.k_chunks - 1u) : 0u;
+  for (uint32_t c = c_lo + warp; c <= c_hi; c += kArgmaxPartsThreads / 32) {
+    const uint32_t x = (uint32_t)((uint64_t)parts.total * c / parts.ctas);  // CTA c's first chunk
+    const uint32_t t = x / parts.k_chunks;
+    if (x % parts.k_chunks == 0 || (int)t < t_lo || (int)t >= t_hi || parts.owner(t * parts.k_chunks) != c - 1) continue;
+    int count;
+    const float* tile = parts.tile(t, count);
+    float v[4];
+    sum_parts<4, 4>(tile, count, row_i, lane * 4, v);
+    const int n = (int)t * kPartCols + lane * 4;
+    if (pairs && n + 3 < vocab) {
+      store4(row + n, v);
+    } else {
+      for (int j = 0; j < 4; ++j)
+        if (n + j < vocab) row[n + j] = __float2bfloat16_rn(v[j]);
+    }
+  }
+  __syncthreads();  // this CTA's columns are complete
+
+  const int lo = t_lo * kPartCols, hi = min(t_hi * kPartCols, vocab);
+  float best = -INFINITY;
+  int best_i = 0x7fffffff;
+  const int vec_end = (reinterpret_cast<uintptr_t>(row + lo) & 15u) == 0 ? lo + ((hi - lo) & ~7) : lo;
+  for (int i = lo + threadIdx.x * 8; i < vec_end; i += kArgmaxPartsThreads * 8) {
+    float v[8];
+    load8(row + i, v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (v[j] > best) { best = v[j]; best_i = i + j; }  // ascending i: the first maximum stays
+  }
+  for (int i = vec_end + threadIdx.x; i < hi; i += kArgmaxPartsThreads) {
+    const float v = __bfloat162float(row[i]);
+    if (v > best || (v == best && i < best_i)) { best = v; best_i = i; }
+  }
+  auto merge = [](float& a, int& ai, float b, int bi) {
+    if (b > a || (b == a && bi < ai)) { a = b; ai = bi; }
+  };
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    merge(best, best_i, __shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, best_i, o));
+  if (lane == 0) { best_s[warp] = best; idx_s[warp] = best_i; }
+  __syncthreads();
+  if (warp == 0) {
+    best = lane < kArgmaxPartsThreads / 32 ? best_s[lane] : -INFINITY;
+    best_i = lane < kArgmaxPartsThreads / 32 ? idx_s[lane] : 0x7fffffff;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      merge(best, best_i, __shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, best_i, o));
+    if (lane == 0) {
+      uint32_t dst_b, dst_i;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(dst_b) : "r"((uint32_t)__cvta_generic_to_shared(rank_best + rank)));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(dst_i) : "r"((uint32_t)__cvta_generic_to_shared(rank_idx + rank)));
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst_b), "f"(best) : "memory");
+      asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(dst_i), "r"(best_i) : "memory");
+    }
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (rank == 0 && threadIdx.x == 0) {
+    best = -INFINITY;
+    best_i = 0x7fffffff;
+    for (int r = 0; r < kArgmaxCluster; ++r) merge(best, best_i, rank_best[r], rank_idx[r]);
+    out[row_i] = best_i == 0x7fffffff ? 0 : best_i;
+  }
+}
+
 template <typename Kern, typename... Args>
 int launch(const char* what, Kern kern, dim3 grid, dim3 block, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg{};
@@ -289,6 +510,93 @@ int ia_llama_argmax(const void* logits, int64_t row_stride, int n_rows, int voca
   const dim3 grid((unsigned)n_rows), block(kArgmaxThreads);
   return launch("llama_argmax_kernel", llama_argmax_kernel, grid, block, (cudaStream_t)stream,
                 static_cast<const __nv_bfloat16*>(logits), row_stride, vocab, out);
+}
+
+static int parts_view(const void* parts, int n, int k, PartsView* out) {
+  if (!parts || !aligned16(parts)) return fail(IA_ERR_BAD_ARG, "parts: null or not 16-byte aligned");
+  if (n <= 0 || k <= 0) return fail(IA_ERR_BAD_ARG, "parts: n %d, k %d", n, k);
+  const GemmSplit s = gemm_split(n, k);
+  if (s.total == 0) return fail(IA_ERR_UNSUPPORTED, "parts: %d x %d is too large", n, k);
+  *out = PartsView{static_cast<const float*>(parts), (uint32_t)s.k_chunks, (uint32_t)s.total, (uint32_t)s.ctas};
+  return IA_OK;
+}
+
+int ia_llama_add_rmsnorm_parts(void* residual, const void* parts, int k, const void* weight, void* out, int n_rows,
+                               int hidden, float eps, ia_stream_t stream) {
+  if (!residual || !weight || !out) return fail(IA_ERR_BAD_ARG, "add_rmsnorm_parts: null pointer");
+  if (n_rows < 0 || n_rows > kPartRows || hidden <= 0 || hidden % 8 != 0)
+    return fail(IA_ERR_BAD_ARG, "add_rmsnorm_parts: %d rows of %d (a multiple of 8)", n_rows, hidden);
+  if (!aligned16(residual) || !aligned16(weight) || !aligned16(out))
+    return fail(IA_ERR_BAD_ARG, "add_rmsnorm_parts: pointers must be 16-byte aligned");
+  PartsView v;
+  if (int s = parts_view(parts, hidden, k, &v)) return s;
+  if (n_rows == 0) return IA_OK;
+  auto* r = static_cast<__nv_bfloat16*>(residual);
+  auto* w = static_cast<const __nv_bfloat16*>(weight);
+  auto* o = static_cast<__nv_bfloat16*>(out);
+  const char* what = "llama_add_rmsnorm_parts_kernel";
+  const dim3 grid((unsigned)n_rows), block(kPartNormThreads);
+  cudaStream_t st = (cudaStream_t)stream;
+  switch ((hidden + kPartNormThreads * 8 - 1) / (kPartNormThreads * 8)) {
+    case 1: return launch(what, llama_add_rmsnorm_parts_kernel<1>, grid, block, st, r, v, w, o, hidden, eps);
+    case 2: return launch(what, llama_add_rmsnorm_parts_kernel<2>, grid, block, st, r, v, w, o, hidden, eps);
+    case 3:
+    case 4: return launch(what, llama_add_rmsnorm_parts_kernel<4>, grid, block, st, r, v, w, o, hidden, eps);
+    default: return fail(IA_ERR_UNSUPPORTED, "add_rmsnorm_parts: hidden size %d above %d", hidden, kPartNormThreads * 32);
+  }
+}
+
+int ia_llama_rope_append_parts(const void* parts, int k, const void* cos_table, const void* sin_table, int max_pos,
+                               const int32_t* seq_lens, void* k_cache, void* v_cache, int64_t cache_seq_stride,
+                               int64_t cache_head_stride, int cache_len, void* q_out, int batch, int n_q_heads,
+                               int n_kv_heads, int head_dim, ia_stream_t stream) {
+  if (!cos_table || !sin_table || !seq_lens || !k_cache || !v_cache || !q_out)
+    return fail(IA_ERR_BAD_ARG, "rope_append_parts: null pointer");
+  if (batch < 0 || batch > kPartRows || n_q_heads <= 0 || n_kv_heads <= 0 || max_pos <= 0 || cache_len <= 0)
+    return fail(IA_ERR_BAD_ARG, "rope_append_parts: batch %d, heads %d/%d, %d positions, cache of %d", batch, n_q_heads,
+                n_kv_heads, max_pos, cache_len);
+  if (head_dim <= 0 || head_dim % 8 != 0 || head_dim > 2048)
+    return fail(IA_ERR_UNSUPPORTED, "rope_append_parts: head_dim %d (a multiple of 8, at most 2048)", head_dim);
+  if (cache_head_stride < (int64_t)cache_len * head_dim || cache_head_stride % 4 != 0 || cache_seq_stride % 4 != 0)
+    return fail(IA_ERR_BAD_ARG, "rope_append_parts: cache strides %lld, %lld for %d rows of %d", (long long)cache_seq_stride,
+                (long long)cache_head_stride, cache_len, head_dim);
+  if ((reinterpret_cast<uintptr_t>(cos_table) | reinterpret_cast<uintptr_t>(sin_table) |
+       reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache) | reinterpret_cast<uintptr_t>(q_out)) & 7u)
+    return fail(IA_ERR_BAD_ARG, "rope_append_parts: pointers must be 8-byte aligned");
+  const int64_t n = (int64_t)(n_q_heads + 2 * n_kv_heads) * head_dim;
+  if (n > 0x7fffffff) return fail(IA_ERR_UNSUPPORTED, "rope_append_parts: %lld columns", (long long)n);
+  PartsView v;
+  if (int s = parts_view(parts, (int)n, k, &v)) return s;
+  if (batch == 0) return IA_OK;
+  const dim3 grid((unsigned)ceil_div64((int64_t)batch * (n / 8), 128)), block(128);
+  return launch("llama_rope_append_parts_kernel", llama_rope_append_parts_kernel, grid, block, (cudaStream_t)stream, v,
+                static_cast<const __nv_bfloat16*>(cos_table), static_cast<const __nv_bfloat16*>(sin_table), max_pos,
+                seq_lens, static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), cache_seq_stride,
+                cache_head_stride, cache_len, static_cast<__nv_bfloat16*>(q_out), batch, n_q_heads, n_kv_heads, head_dim);
+}
+
+int ia_llama_silu_mul_parts(const void* parts, int k, void* out, int n_rows, int intermediate, ia_stream_t stream) {
+  if (!out || !aligned16(out)) return fail(IA_ERR_BAD_ARG, "silu_mul_parts: null or misaligned out");
+  if (n_rows < 0 || n_rows > kPartRows || intermediate <= 0 || intermediate % 8 != 0 || intermediate > 0x3fffffff)
+    return fail(IA_ERR_BAD_ARG, "silu_mul_parts: %d rows of %d (a multiple of 8)", n_rows, intermediate);
+  PartsView v;
+  if (int s = parts_view(parts, 2 * intermediate, k, &v)) return s;
+  if (n_rows == 0) return IA_OK;
+  const dim3 grid((unsigned)ceil_div64((int64_t)n_rows * (intermediate / 8), 256)), block(256);
+  return launch("llama_silu_mul_parts_kernel", llama_silu_mul_parts_kernel, grid, block, (cudaStream_t)stream, v,
+                static_cast<__nv_bfloat16*>(out), n_rows, intermediate);
+}
+
+int ia_llama_argmax_parts(const void* parts, int k, void* logits, int n_rows, int vocab, int64_t* out,
+                          ia_stream_t stream) {
+  if (!logits || !out || (reinterpret_cast<uintptr_t>(logits) & 7u)) return fail(IA_ERR_BAD_ARG, "argmax_parts: null or misaligned pointer");
+  if (n_rows < 0 || n_rows > kPartRows || vocab <= 0) return fail(IA_ERR_BAD_ARG, "argmax_parts: %d rows of %d", n_rows, vocab);
+  PartsView v;
+  if (int s = parts_view(parts, vocab, k, &v)) return s;
+  if (n_rows == 0) return IA_OK;
+  const dim3 grid((unsigned)(n_rows * kArgmaxCluster)), block(kArgmaxPartsThreads);
+  return launch("llama_argmax_parts_kernel", llama_argmax_parts_kernel, grid, block, (cudaStream_t)stream, v,
+                static_cast<__nv_bfloat16*>(logits), vocab, out);
 }
 
 }  // extern "C"

@@ -29,12 +29,12 @@
 
 #include <cuda.h>  // CUtensorMap (types only; the encoder is fetched through the runtime)
 
-#include "ia_common.cuh"
+#include "gemm_parts.cuh"
 
 namespace ia {
 namespace {
 
-constexpr int kBM = 32, kBN = 128, kBK = 64;
+constexpr int kBM = 32, kBN = kPartCols, kBK = kPartChunk;
 constexpr int kWBytes = kBN * kBK * 2, kXBytes = kBM * kBK * 2, kStageBytes = kWBytes + kXBytes;
 constexpr int kSlotFloats = kBM * kBN;  // one fp32 partial tile
 constexpr uint32_t kWaitPolls = 1u << 22;  // polls of a few tens of cycles: some tens of milliseconds
@@ -85,6 +85,22 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     if (mbar_test(bar, parity)) return true;
   return false;
 }
+// The same for waits that take microseconds and whose end nothing urgent follows: try_wait parks the warp, which
+// leaves its scheduler to the warps that issue copies and MMAs.
+__device__ __forceinline__ bool mbar_wait_parked(uint64_t* bar, uint32_t parity) {
+  for (uint32_t i = 0; i < kWaitPolls; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    if (ok != 0) return true;
+  }
+  return false;
+}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
@@ -120,13 +136,15 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
 }
 // instruction descriptor of kind::f16: fp32 accumulate (bit 4), bf16 A and B (bits 7, 10), both K-major,
 // N >> 3 at bit 17, M >> 4 at bit 24
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kBM >> 3) << 17) | ((uint32_t)(kBN >> 4) << 24);
+template <int N>
+constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kBN >> 4) << 24);
 
+template <int N>
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(kIdesc), "r"(accumulate)
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(kIdesc<N>), "r"(accumulate)
       : "memory");
 }
 // the mbarrier gets one arrival when every MMA issued so far by this thread has completed
@@ -136,6 +154,19 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// 32 lanes x 16 columns of fp32: thread t of the warp gets lane (base lane + t), columns [col, col + 16)
+__device__ __forceinline__ void tmem_load_16(uint32_t taddr, float (&v)[16]) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
 // 32 lanes x 32 columns of fp32: thread t of the warp gets lane (base lane + t), columns [col, col + 32)
 __device__ __forceinline__ void tmem_load_32(uint32_t taddr, float (&v)[32]) {
   uint32_t r[32];
@@ -286,7 +317,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) llama_skinny_gemm_tc_kernel(con
         for (int j = 0; j < n; ++j) {
 #pragma unroll
           for (int kk = 0; kk < kBK / 16; ++kk)  // 16 columns = 32 bytes further along K inside the swizzled row
-            umma_bf16(d_tmem, a_desc + (uint64_t)(kk * 2), b_desc + (uint64_t)(kk * 2),
+            umma_bf16<kBM>(d_tmem, a_desc + (uint64_t)(kk * 2), b_desc + (uint64_t)(kk * 2),
                       (first && j == 0 && kk == 0) ? 0u : 1u);
           a_desc += kWBytes >> 4;
           b_desc += kXBytes >> 4;
@@ -395,6 +426,218 @@ __global__ void __launch_bounds__(kTcThreads, 1) llama_skinny_gemm_tc_kernel(con
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
 }
 
+// ---- row-major weights, partial sums left to the consumer ------------------------------------------
+// The projections of the decode step as the step runs them.  The kernel above wants W packed and finishes the tiles
+// it splits itself: park, fence, count, and the last CTA adds - 5 us at the end of a 10 us matrix.  Here W is read as
+// the model holds it (boxes of 64 columns x 128 rows; a ring stage is two or four of them
+// side by side) and a CTA writes what it has of a tile as fp32 into slot cta + tile (both only step by one from a segment to
+// the next, so the sum numbers the segments) and is done.  The kernel that reads the projection next - norm, rotary
+// embedding, SiLU, arg-max - adds the slots of its columns in CTA order (PartsView): no counters, no atomics, the
+// same sum on every run, and one rounding to bf16 where a finished output would have had it.
+// DIRECT: tiles that lie inside one CTA's range are written to `out` in bf16 (the lm head: 854 of 1002 tiles), the
+// consumer completes the others.
+// Bounded by HBM: W once.  W does not depend on the kernel before it on the stream, so the ring is filled (200 KB per
+// SM, 30 MB on the chip) while that kernel still runs; with library GEMMs the short kernels between two projections
+// leave HBM idle for 3 to 6 us each.  Chains of gate/up, SiLU, down, norm at Llama-3-8B sizes (352 MB of weights, 53 us
+// at the HBM rate), one row, this kernel / torch.mm with the same short kernels: 64.8 / 69.7 us; o, norm: 12.0 / 16.1.
+// What is left is some 4 us per kernel boundary.
+// Stages: an iteration of the MMA thread costs 0.3 us and 0.3 us per chunk whatever the copies (one 3-D copy per
+// stage, and two or four accumulators, measured the same), so one chunk per stage is too little (88 us per chain),
+// two give 67, four 64.8 (three stages of 72 KB).  Asking the chunks behind the ring into L2 while the kernel waits made the
+// step slower (four layers 695 -> 711 / 718 / 729 us with 8 / 16 / 32 chunks ahead).
+// Sixteen rows: a 32-row form measured 71.0 against 75.8 us (MLP chain), 13.4 against 12.2 (o, norm) and 170 against 166
+// (lm head), 2.5 % of the batch-32 step; library results at 32 rows differ from it by up to 13 % in single rows (it
+// is the closer one to 64-bit sums: 1.2e-2 over all logits, the library 1.3e-2 to 2.7e-2), and it was not kept.
+struct StreamParams {
+  CUtensorMap tm_w, tm_x;
+  __nv_bfloat16* out;  // DIRECT only
+  float* slots;        // [grid + n_tiles][kPartRows][kBN]
+  int* status;
+  int M, N;
+  int k_chunks, total_chunks;
+};
+struct StreamRing {
+  static constexpr int chunk_x = kPartRows * kBK * 2;
+  static constexpr int cps = 4;  // chunks per stage
+  static constexpr int stage_bytes = cps * (kWBytes + chunk_x);
+  static constexpr int stages = (217 * 1024) / stage_bytes;
+  static constexpr size_t smem = (size_t)stages * stage_bytes + 1024;
+};
+
+template <bool DIRECT>
+__global__ void __launch_bounds__(kTcThreads, 1) llama_stream_gemm_kernel(const __grid_constant__ StreamParams p) {
+  using R = StreamRing;
+  constexpr int MB = kPartRows;  // token rows of the MMA
+  constexpr int kStages = R::stages, CPS = R::cps;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* stage_base =
+      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ uint64_t full_bar[kStages], empty_bar[kStages], acc_full[2], acc_empty[2];
+  __shared__ uint32_t tmem_base_s;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int P = gridDim.x, cta = blockIdx.x;
+  const int T = p.total_chunks, KC = p.k_chunks;
+  const int c0 = (int)((int64_t)T * cta / P), c1 = (int)((int64_t)T * (cta + 1) / P);
+
+  // the producer lane owns the barriers and has W on its way before the CTA's set-up barrier
+  StageWalk w(c0, c1, KC);
+  int w_tile = c0 / KC;
+  auto load_w = [&](int n, unsigned char* st, uint64_t* bar) {
+    for (int j = 0; j < n; ++j) tma_load_2d(st + j * kWBytes, &p.tm_w, (w.kc + j) * kBK, w_tile * kBN, bar);
+  };
+  auto load_x = [&](int n, int kc, unsigned char* st, uint64_t* bar) {
+    for (int j = 0; j < n; ++j) tma_load_2d(st + CPS * kWBytes + j * R::chunk_x, &p.tm_x, (kc + j) * kBK, 0, bar);
+  };
+  auto step_w = [&](int n) {
+    w.advance(n);
+    if (w.kc == 0) ++w_tile;
+  };
+  int primed = 0;
+  if (tid == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_w) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_x) : "memory");
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);  // one tcgen05.commit
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);   // one tcgen05.commit
+      mbar_init(&acc_empty[b], 4);  // one lane of each epilogue warp
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (; primed < kStages && !w.done(); ++primed) {
+      const int n = w.template len<CPS>();
+      mbar_expect_tx(&full_bar[primed], (uint32_t)n * kWBytes);
+      load_w(n, stage_base + (size_t)primed * R::stage_bytes, &full_bar[primed]);
+      step_w(n);
+    }
+  }
+  __syncwarp();
+  if (warp == 1) {  // the whole warp allocates; the base address lands in shared memory
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)),
+                 "r"(kTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_s;
+  grid_launch_dependents();
+
+  if (warp == 0) {
+    if (lane == 0) {
+      grid_dependency_wait();
+      StageWalk x(c0, c1, KC);
+      for (int i = 0; i < primed; ++i) {
+        const int n = x.template len<CPS>();
+        mbar_arrive_expect_tx(&full_bar[i], (uint32_t)(n * R::chunk_x));
+        load_x(n, x.kc, stage_base + (size_t)i * R::stage_bytes, &full_bar[i]);
+        x.advance(n);
+      }
+      bool alive = true;
+      int stage = 0, parity = 0;  // of the empty barrier: use u of a stage waits for the release of use u - 1
+      for (; !w.done();) {
+        if (alive && !mbar_wait(&empty_bar[stage], (uint32_t)parity)) {
+          alive = false;
+          atomicOr(p.status, DEV_STATUS_GEMM_WAIT_TIMEOUT);
+        }
+        const int n = w.template len<CPS>();
+        unsigned char* st = stage_base + (size_t)stage * R::stage_bytes;
+        mbar_arrive_expect_tx(&full_bar[stage], (uint32_t)(n * (kWBytes + R::chunk_x)));
+        load_w(n, st, &full_bar[stage]);
+        load_x(n, w.kc, st, &full_bar[stage]);
+        step_w(n);
+        if (++stage == kStages) { stage = 0; parity ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      bool alive = true;
+      int seg = 0, stage = 0, parity = 0;
+      StageWalk m(c0, c1, KC);
+      while (!m.done()) {
+        const int n = m.template len<CPS>();
+        const bool first = m.starts_tile_or_range(c0);
+        if (first) {
+          const int buf = seg & 1, use = seg >> 1;
+          if (use > 0 && alive && !mbar_wait(&acc_empty[buf], (uint32_t)((use - 1) & 1))) {
+            alive = false;
+            atomicOr(p.status, DEV_STATUS_GEMM_WAIT_TIMEOUT);
+          }
+          ++seg;
+        }
+        const int buf = (seg - 1) & 1;
+        if (alive && !mbar_wait(&full_bar[stage], (uint32_t)parity)) {
+          alive = false;
+          atomicOr(p.status, DEV_STATUS_GEMM_WAIT_TIMEOUT);
+        }
+        tc_fence_after();
+        const uint32_t st = smem_u32(stage_base + (size_t)stage * R::stage_bytes);
+        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * MB);
+        uint64_t a_desc = umma_desc(st), b_desc = umma_desc(st + CPS * kWBytes);
+        for (int j = 0; j < n; ++j) {
+#pragma unroll
+          for (int kk = 0; kk < kBK / 16; ++kk)
+            umma_bf16<MB>(d_tmem, a_desc + (uint64_t)(kk * 2), b_desc + (uint64_t)(kk * 2),
+                          (first && j == 0 && kk == 0) ? 0u : 1u);
+          a_desc += kWBytes >> 4;
+          b_desc += R::chunk_x >> 4;
+        }
+        umma_commit(&empty_bar[stage]);
+        m.advance(n);
+        if (m.kc == 0 || m.done()) umma_commit(&acc_full[buf]);
+        if (++stage == kStages) { stage = 0; parity ^= 1; }
+      }
+    }
+  } else {
+    grid_dependency_wait();  // the slots and the output may still be read by earlier kernels
+    const int q = warp & 3;       // TMEM lane quarter this warp may read
+    const int r = q * 32 + lane;  // row of the tile (= row of W) held by this thread
+    bool alive = true;
+    int seg = 0, from = c0, tile = c0 / KC;
+    while (from < c1) {
+      const int t_lo = tile * KC, t_hi = t_lo + KC;
+      const int to = t_hi < c1 ? t_hi : c1;
+      const int buf = seg & 1, use = seg >> 1;
+      if (alive && !mbar_wait_parked(&acc_full[buf], (uint32_t)(use & 1))) {
+        alive = false;
+        if (lane == 0) atomicOr(p.status, DEV_STATUS_GEMM_WAIT_TIMEOUT);
+      }
+      tc_fence_after();
+      float v[MB];
+      const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * MB);
+      tmem_load_16(acc, v);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[buf]);  // the MMA warp may overwrite this buffer
+      if (DIRECT && from == t_lo && to == t_hi) {
+        const int n = tile * kBN + r;
+        if (n < p.N) {
+#pragma unroll
+          for (int m = 0; m < MB; ++m)
+            if (m < p.M) p.out[(int64_t)m * p.N + n] = __float2bfloat16_rn(v[m]);
+        }
+      } else {
+        float* slot = p.slots + (int64_t)(cta + tile) * (kPartRows * kBN) + r;
+#pragma unroll
+        for (int m = 0; m < MB; ++m)
+          if (m < p.M) slot[m * kBN] = v[m];
+      }
+      from = to;
+      ++tile;
+      ++seg;
+    }
+  }
+  // everyone meets here; then the allocating warp returns the tensor memory
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+}
+
 // Row-major W [N, K] -> the stream the GEMM reads: for every (128-row tile, 64-column chunk), K fastest, the
 // 16 KB shared-memory image of that chunk (rows of 128 bytes, 16-byte piece c of row r at c ^ (r & 7), rows and
 // columns past the matrix zero).  One thread per 16-byte piece of the output.
@@ -450,6 +693,15 @@ template <int CPS> int launch_tc(const GemmParams& p, int grid, cudaStream_t str
   e = launch_overlapped(kern, (unsigned)grid, (unsigned)kTcThreads, TcRing<CPS>::smem, stream, p);
   if (e != cudaSuccess) return fail(IA_ERR_LAUNCH, "llama_skinny_gemm_tc_kernel: %s", cudaGetErrorString(e));
   return check_launch("llama_skinny_gemm_tc_kernel");
+}
+
+template <bool DIRECT> int launch_stream(const StreamParams& p, int grid, cudaStream_t stream) {
+  auto kern = llama_stream_gemm_kernel<DIRECT>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)StreamRing::smem);
+  if (e != cudaSuccess) return fail(IA_ERR_LAUNCH, "stream_gemm: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  e = launch_overlapped(kern, (unsigned)grid, (unsigned)kTcThreads, StreamRing::smem, stream, p);
+  if (e != cudaSuccess) return fail(IA_ERR_LAUNCH, "llama_stream_gemm_kernel: %s", cudaGetErrorString(e));
+  return check_launch("llama_stream_gemm_kernel");
 }
 
 int grid_for(int64_t total_chunks) {
@@ -529,6 +781,39 @@ int ia_llama_gemm(const void* x, const void* w, void* out, int m, int n, int k, 
     case 2: return launch_tc<2>(p, grid, (cudaStream_t)stream);
     default: return launch_tc<4>(p, grid, (cudaStream_t)stream);
   }
+}
+
+int ia_llama_gemm_parts(const void* x, const void* w, void* out, int m, int n, int k, void* parts, int64_t parts_bytes,
+                        ia_stream_t stream) {
+  if (!x || !w || !parts) return fail(IA_ERR_BAD_ARG, "gemm_parts: null pointer");
+  if (m < 0 || m > kPartRows) return fail(IA_ERR_UNSUPPORTED, "gemm_parts: %d rows (at most %d)", m, kPartRows);
+  if (n <= 0 || k <= 0 || k % 8 != 0) return fail(IA_ERR_BAD_ARG, "gemm_parts: n %d, k %d (a multiple of 8)", n, k);
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(parts)) & 15u)
+    return fail(IA_ERR_BAD_ARG, "gemm_parts: x, w and the parts must be 16-byte aligned");
+  if (reinterpret_cast<uintptr_t>(out) & 1u) return fail(IA_ERR_BAD_ARG, "gemm_parts: out must be 2-byte aligned");
+  const GemmSplit split = gemm_split(n, k);
+  if (split.total == 0) return fail(IA_ERR_UNSUPPORTED, "gemm_parts: %d x %d is too large", n, k);
+  if (parts_bytes < ia_llama_gemm_parts_bytes(n, k))
+    return fail(IA_ERR_BAD_ARG, "gemm_parts: parts of %lld bytes, need %lld", (long long)parts_bytes,
+                (long long)ia_llama_gemm_parts_bytes(n, k));
+  if (m == 0) return IA_OK;
+  StreamParams p{};
+  p.out = static_cast<__nv_bfloat16*>(out);
+  p.slots = static_cast<float*>(parts);
+  p.M = m; p.N = n;
+  p.k_chunks = split.k_chunks;
+  p.total_chunks = split.total;
+  p.status = device_status_address();
+  if (p.status == nullptr) return IA_ERR_LAUNCH;
+  if (int s = encode_bf16(&p.tm_w, w, n, k, kBN, CU_TENSOR_MAP_L2_PROMOTION_L2_256B)) return s;
+  if (int s = encode_bf16(&p.tm_x, x, m, k, kPartRows, CU_TENSOR_MAP_L2_PROMOTION_L2_128B)) return s;
+  cudaStream_t st = (cudaStream_t)stream;
+  return out ? launch_stream<true>(p, split.ctas, st) : launch_stream<false>(p, split.ctas, st);
+}
+
+int64_t ia_llama_gemm_parts_bytes(int n, int k) {
+  const GemmSplit s = gemm_split(n, k);
+  return s.total == 0 ? 0 : (int64_t)(s.ctas + (n + kBN - 1) / kBN) * (kPartRows * kBN) * 4;
 }
 
 }  // extern "C"

@@ -10,9 +10,9 @@ static cache, as ten launches per layer:
     add+RMSNorm | QKV GEMM | RoPE+cache append | block selection | sparse attention
     | O GEMM | add+RMSNorm | gate/up GEMM | SiLU*up | down GEMM
 
-The GEMMs run on concatenated weights through ``torch.mm`` (cuBLAS) or, on request,
-``csrc/skinny_gemm.cu`` (a tcgen05 weight-streaming kernel for batches of at most
-32 rows); everything else is ``csrc/llama_step.cu`` and the attention kernels, keeping the
+For batches of at most 16 rows the GEMMs run on ``csrc/skinny_gemm.cu`` (a tcgen05 kernel that streams the
+weights as the model holds them and leaves partial sums to the element-wise kernel that follows); larger batches
+and ``own_gemm="none"`` use ``torch.mm`` (cuBLAS) on the same concatenated weights.  Everything else is ``csrc/llama_step.cu`` and the attention kernels, keeping the
 bf16 rounding points of ``transformers.models.llama.modeling_llama`` so that the
 fused and the module-by-module step agree up to fp32 summation order.
 """
@@ -136,13 +136,16 @@ class FusedLlamaStep:
 
     def __init__(self, model, cache, attention, seq_lens: torch.Tensor, cache_len: int,
                  own_gemm: Optional[str] = None):
-        # own_gemm: which projections run on this library's GEMM kernel instead of torch.mm
-        # (cuBLAS): "all", "none" or a comma-separated subset of PROJECTIONS.  None reads
-        # INTERATTN_B200_LLAMA_GEMM, default "none" (see _linear).  Batches above 32 rows always
-        # use torch.mm.
+        # own_gemm: None reads INTERATTN_B200_LLAMA_GEMM; when that is unset too, batches of at most 16 rows
+        # stream all projections (see _stream_step).  A name pins the form: "none" = torch.mm (cuBLAS), "all" or a
+        # comma-separated subset of PROJECTIONS = those on the packed-weight kernel, the others on torch.mm.
+        # Batches above 32 rows always use torch.mm.
         import os
         if own_gemm is None:
-            own_gemm = os.environ.get("INTERATTN_B200_LLAMA_GEMM", "none")
+            own_gemm = os.environ.get("INTERATTN_B200_LLAMA_GEMM")
+        streaming = own_gemm is None
+        if streaming:
+            own_gemm = "none"
         if own_gemm == "all":
             own = set(self.PROJECTIONS)
         elif own_gemm in ("none", "cublas", ""):
@@ -195,19 +198,82 @@ class FusedLlamaStep:
             if "lm_head" in self.own_gemm:
                 self.lm_head = PackedWeight(self.lm_head)
             torch.cuda.synchronize(dev)
+        self.parts = self._stream_parts() if streaming and 0 < b <= 16 else None
+
+    def _stream_parts(self):
+        """Scratch of the streamed projections (one buffer: each is consumed before the next is written), or None
+        when a size or an address does not suit those kernels and the step stays on torch.mm."""
+        hidden, inter = int(self.x.shape[1]), int(self.act.shape[1])
+        if hidden % 8 or hidden > 16384 or inter % 8 or self.d % 8:
+            return None
+        weights = [self.lm_head] + [L[n] for L in self.layers for n in ("w_qkv", "w_o", "w_gu", "w_down")]
+        others = [self.final_norm, self.cos, self.sin] + [L[n] for L in self.layers for n in ("norm1", "norm2", "k", "v")]
+        if any(not t.is_cuda or t.dtype != torch.bfloat16 or not t.is_contiguous() or t.data_ptr() % 16
+               for t in weights + others):
+            return None
+        size = _lib.load().ia_llama_gemm_parts_bytes
+        need = [int(size(int(w.shape[0]), int(w.shape[1]))) for w in weights]
+        return torch.empty(max(need), dtype=torch.uint8, device=self.x.device) if min(need) > 0 else None
 
     def _linear(self, x: torch.Tensor, w, out: torch.Tensor) -> torch.Tensor:
-        """nn.Linear without bias.  Which kernel: back to back on its own, this library's kernel
-        matches cuBLAS at 32 rows and passes it on the widest shape (lm head, 6.6 against 6.5
-        TB/s); inside the captured Llama-3-8B step its longer start-up and partial-tile tail
-        cost about 7 us per projection (7.6 against 6.7 ms per step with every projection on
-        it), so cuBLAS is the default and the kernel is opt-in."""
+        """nn.Linear without bias, where the projections are not streamed.  Back to back on its own, the
+        packed-weight kernel matches cuBLAS at 32 rows and passes it on the widest shape (lm head, 6.6 against 6.5
+        TB/s); inside the step its longer start-up and partial-tile tail cost about 7 us per projection, so it
+        runs on request only."""
         if isinstance(w, PackedWeight):
             return gemm(x, w, out, self.gemm_ws)
         return torch.mm(x, w.t(), out=out)
 
+    def _stream_step(self, tokens: torch.Tensor) -> None:
+        """The step with every projection streamed (``ia_llama_gemm_parts``): weights start to arrive while the kernel
+        before still runs, and the element-wise kernels add up the partial sums.  Four full-size layers of
+        Llama-3-8B: one sequence 750 -> 679 us, 8 sequences 782 -> 727, 16 sequences 899 -> 851."""
+        lib, check, stream, b = _lib.load(), _lib.check, _stream(), self.x.shape[0]
+        parts, parts_bytes = self.parts.data_ptr(), self.parts.numel()
+        x, h, q, act, hidden, inter = (self.x.data_ptr(), self.h.data_ptr(), self.q.data_ptr(), self.act.data_ptr(),
+                                       self.x.shape[1], self.act.shape[1])
+        cos, sin, max_pos, seq_lens = self.cos.data_ptr(), self.sin.data_ptr(), self.cos.shape[0], self.seq_lens.data_ptr()
+
+        def gemm_parts(src, w, out=None):
+            n, k = w.shape
+            check(lib.ia_llama_gemm_parts(src, w.data_ptr(), out, b, n, k, parts, parts_bytes, stream))
+            return k
+
+        def add_norm(k, weight):
+            check(lib.ia_llama_add_rmsnorm_parts(x, parts, k, weight.data_ptr(), h, b, hidden, self.eps, stream))
+
+        k = None
+        for L, attn in zip(self.layers, self.attention):
+            if k is None:
+                add_rmsnorm(self.x, None, L["norm1"], self.eps, self.h)
+            else:
+                add_norm(k, L["norm1"])
+            k = gemm_parts(h, L["w_qkv"])
+            k_cache, v_cache = L["k"], L["v"]
+            t = k_cache.shape[2]
+            check(lib.ia_llama_rope_append_parts(parts, k, cos, sin, max_pos, seq_lens, k_cache.data_ptr(),
+                                                 v_cache.data_ptr(), self.hkv * t * self.d, t * self.d, t, q, b, self.hq,
+                                                 self.hkv, self.d, stream))
+            ctx = attn.step(self.q)
+            k = gemm_parts(ctx.data_ptr(), L["w_o"])
+            add_norm(k, L["norm2"])
+            k = gemm_parts(h, L["w_gu"])
+            check(lib.ia_llama_silu_mul_parts(parts, k, act, b, inter, stream))
+            k = gemm_parts(act, L["w_down"])
+        if k is None:
+            add_rmsnorm(self.x, None, self.final_norm, self.eps, self.h)
+        else:
+            add_norm(k, self.final_norm)
+        k = gemm_parts(h, self.lm_head, self.logits.data_ptr())
+        check(lib.ia_llama_argmax_parts(parts, k, self.logits.data_ptr(), b, self.logits.shape[1], tokens.data_ptr(), stream))
+
     @torch.no_grad()
     def step(self, tokens: torch.Tensor) -> torch.Tensor:
+        if self.parts is not None and tokens.is_cuda and tokens.dtype == torch.int64 and tokens.is_contiguous() \
+                and tokens.numel() == self.x.shape[0]:
+            torch.index_select(self.embed, 0, tokens.view(-1), out=self.x)
+            self._stream_step(tokens)
+            return tokens
         b = self.x.shape[0]
         torch.index_select(self.embed, 0, tokens.view(-1), out=self.x)
         delta = None

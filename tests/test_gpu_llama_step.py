@@ -126,6 +126,83 @@ def test_skinny_gemm(m, n, k):
     assert int(ws[: ((n + 127) // 128) * 4].view(torch.int32).abs().sum()) == 0
 
 
+# sizes: fewer chunks than SMs; a tile split over many CTAs; CTAs that own whole tiles; ragged N, K and vocab;
+# one row, an odd number, all sixteen
+@pytest.mark.parametrize("m", [1, 7, 16])
+@pytest.mark.parametrize("n,k", [(512, 512), (1000, 72), (4096, 14336), (136, 20000), (28672, 512), (6144, 4096)])
+def test_streamed_gemm_and_its_consumers(m, n, k):
+    """The consumers of the partial sums against the same kernels on the finished projection (fp32 product of the same
+    inputs, rounded to bf16).  Another summation order moves a projection by at most its fp32 error before the
+    rounding, so results agree but for values that round the other way: a bf16 ulp of the projection."""
+    from interattn_b200 import _lib
+    ls, lib = _step(), _lib.load()
+    g = torch.Generator().manual_seed(m * 7 + n + k)
+    x = torch.randn(m, k, generator=g).to(BF).to(DEV)
+    w = (torch.randn(n, k, generator=g) / k ** 0.5).to(BF).to(DEV)
+    nan = lambda *shape: torch.full(shape, float("nan"), dtype=BF, device=DEV)  # noqa: E731
+    parts = torch.full((lib.ia_llama_gemm_parts_bytes(n, k) // 4,), float("nan"), device=DEV)
+    stream = torch.cuda.current_stream().cuda_stream
+    want32 = x.double() @ w.double().t()
+    want = want32.to(BF)
+
+    def product(out=None):
+        parts.fill_(float("nan"))
+        _lib.check(lib.ia_llama_gemm_parts(x.data_ptr(), w.data_ptr(), None if out is None else out.data_ptr(), m, n, k,
+                                           parts.data_ptr(), parts.numel() * 4, stream))
+
+    def near(got, ref, scale):   # one bf16 ulp of `scale`, plus the fp32 sum's error
+        err = (got.double() - ref.double()).abs()
+        assert bool((err <= 2.0 ** -7 * scale.double().abs() + 1e-3).all()), float(err.max())
+
+    logits, first = nan(m, n), torch.full((m,), -7, dtype=torch.int64, device=DEV)
+    product(logits)
+    _lib.check(lib.ia_llama_argmax_parts(parts.data_ptr(), k, logits.data_ptr(), m, n, first.data_ptr(), stream))
+    torch.cuda.synchronize()
+    err = (logits.double() - want32).abs()
+    assert bool((err <= 2.0 ** -8 * want32.abs() + 1e-3).all()), float(err.max())
+    assert torch.equal(first.cpu(), lo.argmax_first(logits.cpu()))
+
+    if n % 8 == 0 and n <= 16384:
+        res = torch.randn(m, n, generator=g).to(BF).to(DEV)
+        norm = (1 + 0.1 * torch.randn(n, generator=g)).to(BF).to(DEV)
+        ref_res, ref_out, got_res, got_out = res.clone(), nan(m, n), res.clone(), nan(m, n)
+        ls.add_rmsnorm(ref_res, logits, norm, 1e-5, ref_out)
+        product()
+        _lib.check(lib.ia_llama_add_rmsnorm_parts(got_res.data_ptr(), parts.data_ptr(), k, norm.data_ptr(),
+                                                  got_out.data_ptr(), m, n, 1e-5, stream))
+        assert torch.equal(got_res, ref_res)         # the same sums in the same order, the same rounding
+        near(got_out, ref_out, ref_out)
+    if n % 16 == 0:
+        ref, got = nan(m, n // 2), nan(m, n // 2)
+        ls.silu_mul(logits, ref)
+        product()
+        _lib.check(lib.ia_llama_silu_mul_parts(parts.data_ptr(), k, got.data_ptr(), m, n // 2, stream))
+        assert torch.equal(got, ref)
+    for d in (64, 128):
+        heads = n // d
+        if n % d or heads < 4:
+            continue
+        hkv, t = max(1, heads // 6), 48
+        hq = heads - 2 * hkv
+        pos = torch.randint(0, t + 2, (m,), generator=g).to(torch.int32).to(DEV)   # out-of-range rows stay as they are
+        cos, sin = (torch.randn(t, d, generator=g).to(BF).to(DEV) for _ in range(2))
+        ref = [torch.zeros(m, hkv, t, d, dtype=BF, device=DEV) for _ in range(2)] + [torch.zeros(m, hq, d, dtype=BF, device=DEV)]
+        got = [a.clone() for a in ref]
+        ls.rope_append(logits, cos, sin, pos, *ref)
+        product()
+        _lib.check(lib.ia_llama_rope_append_parts(
+            parts.data_ptr(), k, cos.data_ptr(), sin.data_ptr(), t, pos.data_ptr(), got[0].data_ptr(), got[1].data_ptr(),
+            hkv * t * d, t * d, t, got[2].data_ptr(), m, hq, hkv, d, stream))
+        for a, c in zip(got, ref):
+            assert torch.equal(a, c)
+    from interattn_b200 import ops
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    with pytest.raises(ValueError):   # more rows than a slot holds
+        _lib.check(lib.ia_llama_gemm_parts(x.data_ptr(), w.data_ptr(), None, 17, n, k, parts.data_ptr(),
+                                           parts.numel() * 4, stream))
+
+
 def test_bad_arguments_raise():
     ls = _step()
     x = torch.zeros(2, 100, dtype=BF, device=DEV)               # hidden not a multiple of 8
@@ -144,7 +221,8 @@ def test_bad_arguments_raise():
                 torch.zeros(4, 128, dtype=BF, device=DEV), torch.zeros(16, dtype=torch.uint8, device=DEV))
 
 
-@pytest.mark.parametrize("graph,own_gemm", [(False, "none"), (True, "none"), (False, "all"), (True, "w_down,lm_head")])
+@pytest.mark.parametrize("graph,own_gemm", [(False, "none"), (True, "none"), (False, "all"), (True, "w_down,lm_head"),
+                                            (False, None), (True, None)])
 def test_fused_step_matches_the_module_by_module_step(graph, own_gemm):
     """Same weights, same prompts, the same tokens fed at every step: the logits of the fused
     step follow those of the Hugging Face modules around the attention hook."""
