@@ -2022,14 +2022,14 @@ static int launch_kernel(Kern kern, const char* name, const SelectParams& p, int
   return check_launch(name);
 }
 
-// The fused form applies to bf16 pools with head_dim 128, at most eight query rows per kv head, a
+// The fused form applies to bf16 pools, at most eight query rows per kv head, a
 // grid that is resident at once, no exchange with other GPUs, and a ring that holds at least one page
 // per attending warp.  INTERATTN_B200_FUSED=0 / ia_set_fused_step(0) keep the two kernels;
 // INTERATTN_B200_FUSED_WAVES=any lifts the single-wave rule (an experiment switch: measured slower).
 template <typename T, int D, int G, int NG, typename KB, int BOUND>
 static bool try_launch_fused(SelectParams& p, const AttendRequest& ar, int n_pairs, size_t smem, size_t ring_bytes,
                              int resident_ctas, cudaStream_t stream, int* status) {
-  if constexpr (sizeof(T) == 2 && D == 128 && G <= 8) {
+  if constexpr (sizeof(T) == 2 && G <= 8) {
     // One wave only: with more CTAs than resident slots a CTA would hold its SM through the serial
     // phases of the selection while the attention of other pairs waits for a slot (measured: the ragged
     // 70B batch, 512 pairs, 255 us fused against 240 us as two kernels).
@@ -2038,6 +2038,11 @@ static bool try_launch_fused(SelectParams& p, const AttendRequest& ar, int n_pai
       return v != nullptr && strcmp(v, "any") == 0;
     }();
     if (ar.req == nullptr || p.xch.n_ranks > 0 || (n_pairs * p.cluster > resident_ctas && !any_waves)) return false;
+    // head_dim 64: a page is 4 KB in two copies, and a CTA with a pair to itself pulls less than the attention kernel's
+    // 4 warps x 2 CTAs per SM do; one launch wins where a cluster shares the pair.  One kernel / two, us: 64 ragged
+    // pairs (clusters of 2) 19.0 / 20.5, 8 pairs (4) 16.8 / 18.4, 32 pairs of 8 rows (4) 24.1 / 25.1; 128 pairs (1)
+    // 29.7 / 28.0, 192 pairs (1, narrow) 28.8 / 23.8, 256 ragged pairs (1, narrow) 62.3 / 53.3.
+    if (D == 64 && p.cluster == 1) return false;
     const bool off = !fused_step_enabled();
     const ia_geom& g = *ar.geom;
     constexpr size_t kStage = 2 * 16 * D * 2;
@@ -2100,7 +2105,7 @@ static int launch_shaped(SelectParams& p, const AttendRequest& ar, int n_pairs, 
 // rule a sixteenth of them (what ia_suggest_splits assumes).  0: the step will not run as one kernel.
 template <typename T, int D, int G>
 static int fused_step_pages(const SelectParams& p, const AttendRequest& ar, int max_tiles) {
-  if (!(sizeof(T) == 2 && D == 128 && G <= 8) || ar.req == nullptr || p.xch.n_ranks > 0 ||
+  if (!(sizeof(T) == 2 && G <= 8) || ar.req == nullptr || p.xch.n_ranks > 0 ||
       ar.geom->n_pool_pages <= 0 || !fused_step_enabled())
     return 0;
   const int blocks = p.mode == IA_SELECT_TOPK ? min(p.top_k, p.max_blocks) : max_tiles * kTileBlocks / 16;

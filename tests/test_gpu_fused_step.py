@@ -88,6 +88,21 @@ def test_fused_step_matches_selection_and_oracle(cfg, shape, cluster, rep_mode, 
     torch.testing.assert_close(out.float(), two.float(), **TOL)
 
 
+D64_CASES = [
+    DecodeConfig("d64_g1_ragged", "bfloat16", 4, 2, 2, 64, 16, 64, 2, (1, 129, 1000, 0), (15, 16, 17, 40), seed=31),
+    DecodeConfig("d64_g4_block32", "bfloat16", 2, 8, 2, 64, 16, 32, 5, (1000, 333), (3, 40), seed=32),
+    DecodeConfig("d64_g8_long_suffix", "bfloat16", 2, 16, 2, 64, 16, 64, 9, (2311, 7), (300, 5), seed=33),
+    DecodeConfig("d64_g2_no_suffix", "bfloat16", 3, 4, 2, 64, 16, 128, 3, (2000, 129, 128), (0, 0, 0), seed=34),
+]
+
+
+@pytest.mark.parametrize("rep_mode", ["sparse_only", "hybrid"])
+@pytest.mark.parametrize("shape,cluster", [("wide", 2), ("narrow", 2), ("wide", 4), ("wide", 8)])
+@pytest.mark.parametrize("cfg", D64_CASES, ids=lambda c: c.name)
+def test_fused_step_head_dim_64(cfg, shape, cluster, rep_mode, monkeypatch):
+    test_fused_step_matches_selection_and_oracle(cfg, shape, cluster, rep_mode, monkeypatch)
+
+
 def test_switch_between_the_one_kernel_and_the_two_kernel_form(monkeypatch):
     ops = _ops()
     monkeypatch.setenv("INTERATTN_B200_SELECT_CLUSTER", "1")
