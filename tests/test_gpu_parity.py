@@ -602,3 +602,46 @@ def test_streaming_and_direct_summary_kernels_agree(dtype, head_dim, monkeypatch
     full, part = built["stream"]
     assert bool((part.k_max[1, :, :9] == 7.0).all()) and torch.equal(part.k_max[1, :, 9:16], full.k_max[1, :, 9:16])
     assert bool((part.k_max[3, :, :30] == 7.0).all()) and torch.equal(part.k_max[3, :, 30:33], full.k_max[3, :, 30:33])
+
+
+@pytest.mark.parametrize("rep_mode", ["sparse_only", "hybrid"])
+@pytest.mark.parametrize("group", [1, 2, 8])
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("n_splits", [1, 5])
+def test_fp32_attention_tiles_and_dead_rows(n_splits, head_dim, group, rep_mode):
+    """The FMA kernel takes the 16 tokens of a page together: partly live pages at both ends, pages and tiles of
+    representatives with nothing live, an empty sequence, NaN in every dead row.  fp32 sums of a few hundred terms
+    of order one against the oracle's: well inside 1e-5 relative to the largest value."""
+    from oracle.configs import DecodeConfig, make_case
+    from tests.gpu_util import logical_kv, max_blocks_of, oracle_summaries_from_gpu, to_device
+    from interattn_b200 import ops
+    cfg = DecodeConfig("fp32_tiles", "float32", 4, 2 * group, 2, head_dim, 16, 32, 4, (333, 16, 545, 1), (1, 17, 0, 30), seed=51)
+    case = make_case(cfg, spare_pages=2)
+    q, kv = to_device(case)
+    used = torch.zeros(kv.k_pool.shape[0], 16, dtype=torch.bool, device=q.device)
+    for b in range(cfg.batch):
+        n = int(case["seq_lens"][b])
+        for j in range((n + 15) // 16):
+            used[int(kv.block_table[b, j]), : min(16, n - 16 * j)] = True
+    dead = (~used)[:, None, :, None].expand_as(kv.k_pool)
+    kv.k_pool[dead], kv.v_pool[dead] = float("nan"), float("nan")
+    summ = ops.build_summaries(kv, cfg.block_size, max_blocks=max_blocks_of(case))
+    idx, cnt, aux = ops.select_blocks(q, summ, kv.prefix_lens, top_k=cfg.top_k, want=("z",))
+    o, lse = ops.sparse_decode(q, kv, idx, cnt, block_size=cfg.block_size, max_blocks=summ.max_blocks, n_splits=n_splits,
+                               rep_mode=rep_mode, summ=summ, z=aux["z"])
+    got = ops.finalize(o, lse, torch.float32).cpu()
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    for b in range(cfg.batch):
+        plen = int(case["prefix_lens"][b])
+        osum = oracle_summaries_from_gpu(summ, b, plen)
+        k, v = logical_kv(case, b)
+        mask = torch.zeros((2, osum.n_blocks), dtype=torch.bool)
+        for h in range(2):
+            mask[h, idx[b, h, : int(cnt[b, h])].cpu().long()] = True
+        extra = {}
+        if rep_mode == "hybrid":
+            extra = dict(z=aux["z"][b, :, : osum.n_blocks].cpu().reshape(2, group, -1), v_bar=osum.v_bar)
+        want = orc.decode_attention(case["q"][b].reshape(2, group, head_dim).float(), k, v, plen, cfg.block_size, mask,
+                                    rep_mode=rep_mode, **extra)
+        torch.testing.assert_close(got[b].reshape(2, group, head_dim), want, rtol=1e-5, atol=1e-5)
