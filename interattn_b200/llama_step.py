@@ -179,11 +179,15 @@ class FusedLlamaStep:
         self.lm_head = model.lm_head.weight
         b = int(seq_lens.numel())
         dev, h, inter = p0.device, int(cfg.hidden_size), int(cfg.intermediate_size)
+        q_cols, kv_cols = self.hq * self.d, self.hkv * self.d
+        self._layer_shapes = (("norm1", (h,)), ("w_qkv", (q_cols + 2 * kv_cols, h)), ("w_o", (h, q_cols)),
+                              ("norm2", (h,)), ("w_gu", (2 * inter, h)), ("w_down", (h, inter)))
         with torch.no_grad():
             pos = torch.arange(cache_len, device=dev)[None, :]
             cos, sin = core.rotary_emb(torch.empty((1,), dtype=torch.bfloat16, device=dev), pos)
         self.cos, self.sin = cos[0].contiguous(), sin[0].contiguous()
         new = lambda *shape: torch.empty(shape, dtype=torch.bfloat16, device=dev)  # noqa: E731
+        # the streamed form writes neither o, down, qkv nor gu; they are there for a step that has to leave it
         self.x, self.h, self.o, self.down = new(b, h), new(b, h), new(b, h), new(b, h)
         self.qkv, self.q = new(b, (self.hq + 2 * self.hkv) * self.d), new(b, self.hq, self.d)
         self.gu, self.act = new(b, 2 * inter), new(b, inter)
@@ -198,19 +202,45 @@ class FusedLlamaStep:
             if "lm_head" in self.own_gemm:
                 self.lm_head = PackedWeight(self.lm_head)
             torch.cuda.synchronize(dev)
+        self._device_index = self.x.get_device()
         self.parts = self._stream_parts() if streaming and 0 < b <= 16 else None
+
+    def _fits(self, t: torch.Tensor, shape) -> bool:
+        """``t`` is what the streamed kernels take an address for: bf16 rows of this shape on the step's device."""
+        return t.shape == shape and t.dtype is torch.bfloat16 and t.get_device() == self._device_index \
+            and t.is_contiguous() and not t.data_ptr() & 15
+
+    def _layer_fits(self, L) -> bool:
+        """The streamed kernels get addresses only.  Weights and caches may be replaced between steps, so this is asked
+        on every step, like the checks of ``rope_append`` and ``torch.mm`` in the other form."""
+        k = L["k"]
+        cache = (self.x.shape[0], self.hkv, k.shape[2] if k.dim() == 4 else 0, self.d)
+        if not self._fits(k, cache) or not self._fits(L["v"], cache):
+            return False
+        for name, shape in self._layer_shapes:
+            if not self._fits(L[name], shape):
+                return False
+        return True
+
+    def _ends_fit(self) -> bool:
+        """The same for what the layers share."""
+        b, hidden = self.x.shape
+        lens, tables = self.seq_lens, (self.cos.shape[0], self.d)
+        return (lens.dtype is torch.int32 and lens.numel() == b and lens.is_contiguous()
+                and lens.get_device() == self._device_index and self._fits(self.cos, tables)
+                and self._fits(self.sin, tables) and self._fits(self.final_norm, (hidden,))
+                and self._fits(self.lm_head, (self.logits.shape[1], hidden)))
 
     def _stream_parts(self):
         """Scratch of the streamed projections (one buffer: each is consumed before the next is written), or None
-        when a size or an address does not suit those kernels and the step stays on torch.mm."""
+        when a size or an address does not suit those kernels and the step stays on torch.mm, which refuses what is
+        wrong rather than unsuitable."""
         hidden, inter = int(self.x.shape[1]), int(self.act.shape[1])
-        if hidden % 8 or hidden > 16384 or inter % 8 or self.d % 8:
+        if not self.x.is_cuda or hidden % 8 or hidden > 16384 or inter % 8 or self.d % 8:
+            return None
+        if not self._ends_fit() or not all(self._layer_fits(L) for L in self.layers):
             return None
         weights = [self.lm_head] + [L[n] for L in self.layers for n in ("w_qkv", "w_o", "w_gu", "w_down")]
-        others = [self.final_norm, self.cos, self.sin] + [L[n] for L in self.layers for n in ("norm1", "norm2", "k", "v")]
-        if any(not t.is_cuda or t.dtype != torch.bfloat16 or not t.is_contiguous() or t.data_ptr() % 16
-               for t in weights + others):
-            return None
         size = _lib.load().ia_llama_gemm_parts_bytes
         need = [int(size(int(w.shape[0]), int(w.shape[1]))) for w in weights]
         return torch.empty(max(need), dtype=torch.uint8, device=self.x.device) if min(need) > 0 else None
@@ -224,11 +254,15 @@ class FusedLlamaStep:
             return gemm(x, w, out, self.gemm_ws)
         return torch.mm(x, w.t(), out=out)
 
-    def _stream_step(self, tokens: torch.Tensor) -> None:
+    def _stream_step(self, tokens: torch.Tensor) -> bool:
         """The step with every projection streamed (``ia_llama_gemm_parts``): weights start to arrive while the kernel
-        before still runs, and the element-wise kernels add up the partial sums.  Four full-size layers of
-        Llama-3-8B: one sequence 750 -> 679 us, 8 sequences 782 -> 727, 16 sequences 899 -> 851."""
+        before still runs, and the element-wise kernels add up the partial sums.  False: something does not fit (any
+        more), nothing that reads or writes it was launched, and the other form has to take the step from its start.
+        Four full-size layers of Llama-3-8B: one sequence 750 -> 679 us, 8 sequences 782 -> 727, 16 sequences 899 -> 851."""
+        if not self._ends_fit():
+            return False
         lib, check, stream, b = _lib.load(), _lib.check, _stream(), self.x.shape[0]
+        ctx_shape = (b, self.hq * self.d)
         parts, parts_bytes = self.parts.data_ptr(), self.parts.numel()
         x, h, q, act, hidden, inter = (self.x.data_ptr(), self.h.data_ptr(), self.q.data_ptr(), self.act.data_ptr(),
                                        self.x.shape[1], self.act.shape[1])
@@ -244,6 +278,8 @@ class FusedLlamaStep:
 
         k = None
         for L, attn in zip(self.layers, self.attention):
+            if not self._layer_fits(L):
+                return False
             if k is None:
                 add_rmsnorm(self.x, None, L["norm1"], self.eps, self.h)
             else:
@@ -254,7 +290,9 @@ class FusedLlamaStep:
             check(lib.ia_llama_rope_append_parts(parts, k, cos, sin, max_pos, seq_lens, k_cache.data_ptr(),
                                                  v_cache.data_ptr(), self.hkv * t * self.d, t * self.d, t, q, b, self.hq,
                                                  self.hkv, self.d, stream))
-            ctx = attn.step(self.q)
+            ctx = attn.step(self.q).view(ctx_shape)
+            if not self._fits(ctx, ctx_shape):
+                return False
             k = gemm_parts(ctx.data_ptr(), L["w_o"])
             add_norm(k, L["norm2"])
             k = gemm_parts(h, L["w_gu"])
@@ -266,14 +304,15 @@ class FusedLlamaStep:
             add_norm(k, self.final_norm)
         k = gemm_parts(h, self.lm_head, self.logits.data_ptr())
         check(lib.ia_llama_argmax_parts(parts, k, self.logits.data_ptr(), b, self.logits.shape[1], tokens.data_ptr(), stream))
+        return True
 
     @torch.no_grad()
     def step(self, tokens: torch.Tensor) -> torch.Tensor:
-        if self.parts is not None and tokens.is_cuda and tokens.dtype == torch.int64 and tokens.is_contiguous() \
-                and tokens.numel() == self.x.shape[0]:
+        if self.parts is not None and tokens.device == self.x.device and tokens.dtype == torch.int64 \
+                and tokens.is_contiguous() and tokens.numel() == self.x.shape[0]:
             torch.index_select(self.embed, 0, tokens.view(-1), out=self.x)
-            self._stream_step(tokens)
-            return tokens
+            if self._stream_step(tokens):
+                return tokens
         b = self.x.shape[0]
         torch.index_select(self.embed, 0, tokens.view(-1), out=self.x)
         delta = None

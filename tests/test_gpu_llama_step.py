@@ -247,3 +247,25 @@ def test_fused_step_matches_the_module_by_module_step(graph, own_gemm):
                                                     fused_step=True, own_gemm=own_gemm, cuda_graph=True)
         assert st["cuda_graph"] and st["fused_step"]
         assert torch.equal(t_eager, t_graph)
+
+
+@pytest.mark.parametrize("own_gemm", [None, "none"])
+@pytest.mark.parametrize("what", ["batch", "kv_heads", "v_shorter", "int64_lens"])
+def test_a_cache_that_does_not_fit_is_refused(what, own_gemm):
+    """Both forms refuse the step before anything writes to the cache."""
+    pytest.importorskip("transformers")
+    import types
+    from interattn_b200 import llama_decode, llama_step
+    model = llama_decode.build_random_llama("tiny", dtype=BF, device=DEV, seed=3)
+    cfg, b, t = model.config, 3, 64
+    hkv, d = cfg.num_key_value_heads, getattr(cfg, "head_dim", None) or cfg.hidden_size // cfg.num_attention_heads
+    shape = [b - (what == "batch"), hkv - (what == "kv_heads"), t, d]
+    k = torch.zeros(shape, dtype=BF, device=DEV)
+    v = torch.zeros(shape[:2] + [t - 16 * (what == "v_shorter"), d], dtype=BF, device=DEV)
+    lens = torch.full((b,), 40, dtype=torch.int64 if what == "int64_lens" else torch.int32, device=DEV)
+    cache = types.SimpleNamespace(layers=[types.SimpleNamespace(keys=k, values=v)] * cfg.num_hidden_layers)
+    step = llama_step.FusedLlamaStep(model, cache, [None] * cfg.num_hidden_layers, lens, t, own_gemm=own_gemm)
+    with pytest.raises(ValueError):
+        step.step(torch.zeros((b, 1), dtype=torch.int64, device=DEV))
+    torch.cuda.synchronize()
+    assert float(k.abs().sum()) == 0 and float(v.abs().sum()) == 0
