@@ -342,6 +342,8 @@ def _condition_block_decode_output_fused_triton(
     geo.ensure(prompt_len + n_suffix + 1)
     if not (torch.is_tensor(suffix_len_dev) and suffix_len_dev.is_cuda):
         raise ValueError("suffix_len_dev must be a CUDA int32 scalar tensor")
+    if suffix_len_dev.get_device() != cache.get_device():   # the kernels read it where it lies
+        raise ValueError(f"suffix_len_dev is on {suffix_len_dev.device}, the cache on {cache.device}")
     if suffix_len_dev.dtype != torch.int32 or suffix_len_dev.numel() != 1:
         suffix_len_dev = suffix_len_dev.reshape(1).to(torch.int32)
 

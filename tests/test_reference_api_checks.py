@@ -1,0 +1,37 @@
+"""Host-side behaviour of the reference-named calls, without a GPU: tensors that only claim to be on one (fake
+tensors), and a library that records its calls instead of launching anything."""
+
+import pytest
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+
+from interattn_b200 import _lib, ops, reference_api as api
+
+HKV, G, D, BLOCK, PROMPT = 2, 4, 64, 64, 128
+NB = PROMPT // BLOCK
+
+
+def _prefix(device):
+    new = lambda *shape, dtype=torch.bfloat16: torch.empty(shape, dtype=dtype, device=device)  # noqa: E731
+    cache = [new(HKV, PROMPT + 64, D)[:, :PROMPT] for _ in range(2)]
+    slab = (1, HKV, NB, D)
+    summ = ops.BlockSummaries(k_bar=new(*slab, dtype=torch.float32), k_max=new(*slab), k_min=new(*slab),
+                              v_bar=new(*slab), v_norm_max=new(1, HKV, NB, dtype=torch.float32), block_size=BLOCK)
+    geometry = api._CacheGeometry(device, PROMPT)
+    return {"block_valid_counts": new(NB, dtype=torch.int64),
+            "_b200": api._PrefixHandle(*cache, BLOCK, summ, geometry)}
+
+
+@pytest.mark.filterwarnings("ignore:Accessing the data pointer")
+def test_the_suffix_length_lives_on_the_cache_device():
+    """The kernels read the length where it lies, so a scalar of another GPU is refused and not dereferenced."""
+    with FakeTensorMode():
+        prefix = _prefix("cuda:0")
+        q = torch.empty((HKV, G, 1, D), dtype=torch.bfloat16, device="cuda:0")
+        empty = torch.empty((HKV, 0, D), dtype=torch.bfloat16, device="cuda:0")
+        for length in (torch.zeros((), dtype=torch.int32, device="cuda:1"), torch.zeros((1,), dtype=torch.int64, device="cuda:1"),
+                       torch.zeros((), dtype=torch.int32)):
+            with pytest.raises(ValueError, match="suffix_len_dev"):
+                api._condition_block_decode_output_fused_triton(
+                    q_grouped=q, prompt_prefix=prefix, k_suffix=empty, v_suffix=empty, suffix_len_dev=length, eps=None,
+                    top_k=1, page_size=BLOCK, store_selected=False, output_dtype=None, workspace={})
