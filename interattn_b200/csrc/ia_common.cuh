@@ -121,6 +121,16 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 __device__ __forceinline__ void grid_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// ---- start of a thread-block cluster ---------------------------------------------
+// Shared memory of a peer CTA may be touched only once that CTA is known to run.  Every thread of the cluster arrives
+// at the kernel's start and waits before the first remote access; by then the others have long arrived, so the wait
+// costs nothing.
+__device__ __forceinline__ void cluster_arrive_started() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait_started() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 bool overlapped_launch_enabled();
 // the one-kernel layer step may be used (INTERATTN_B200_FUSED, ia_set_fused_step)
 bool fused_step_enabled();

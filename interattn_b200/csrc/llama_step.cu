@@ -330,6 +330,7 @@ constexpr int kArgmaxPartsThreads = 512, kArgmaxCluster = 8;
 __global__ void __cluster_dims__(kArgmaxCluster, 1, 1) __launch_bounds__(kArgmaxPartsThreads)
 llama_argmax_parts_kernel(const PartsView parts, __nv_bfloat16* __restrict__ logits, int vocab,
                           int64_t* __restrict__ out) {
+  cluster_arrive_started();
   grid_launch_dependents();
   grid_dependency_wait();
   __shared__ float best_s[kArgmaxPartsThreads / 32];
@@ -387,6 +388,7 @@ llama_argmax_parts_kernel(const PartsView parts, __nv_bfloat16* __restrict__ log
     merge(best, best_i, __shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, best_i, o));
   if (lane == 0) { best_s[warp] = best; idx_s[warp] = best_i; }
   __syncthreads();
+  cluster_wait_started();  // rank 0 runs: its shared memory may be written (a rank without tiles is here at once)
   if (warp == 0) {
     best = lane < kArgmaxPartsThreads / 32 ? best_s[lane] : -INFINITY;
     best_i = lane < kArgmaxPartsThreads / 32 ? idx_s[lane] : 0x7fffffff;

@@ -249,6 +249,32 @@ def test_fused_step_matches_the_module_by_module_step(graph, own_gemm):
         assert torch.equal(t_eager, t_graph)
 
 
+@pytest.mark.parametrize("n", [8, 130, 1024, 1100])
+def test_streamed_argmax_where_cluster_ranks_have_no_tile(n):
+    """Eight CTAs share a row: up to seven tiles of 128 columns some of them only hand over "nothing".  Repeated with
+    other inputs back to back, so that clusters of several launches start at different times.  Exact: the logits the
+    kernel completed decide."""
+    from interattn_b200 import _lib, ops
+    lib, m, k = _lib.load(), 16, 192
+    g = torch.Generator(device=DEV).manual_seed(n)
+    parts = torch.empty(lib.ia_llama_gemm_parts_bytes(n, k), dtype=torch.uint8, device=DEV)
+    stream = torch.cuda.current_stream().cuda_stream
+    kept = []
+    for _ in range(20):
+        x = torch.randn(m, k, generator=g, device=DEV).to(BF)
+        w = torch.randn(n, k, generator=g, device=DEV).to(BF)
+        logits = torch.empty(m, n, dtype=BF, device=DEV)
+        first = torch.full((m,), -7, dtype=torch.int64, device=DEV)
+        _lib.check(lib.ia_llama_gemm_parts(x.data_ptr(), w.data_ptr(), logits.data_ptr(), m, n, k, parts.data_ptr(),
+                                           parts.numel(), stream))
+        _lib.check(lib.ia_llama_argmax_parts(parts.data_ptr(), k, logits.data_ptr(), m, n, first.data_ptr(), stream))
+        kept.append((x, w, logits, first))
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    for x, w, logits, first in kept:
+        assert torch.equal(first.cpu(), lo.argmax_first(logits.cpu()))
+
+
 @pytest.mark.parametrize("own_gemm", [None, "none"])
 @pytest.mark.parametrize("what", ["batch", "kv_heads", "v_shorter", "int64_lens"])
 def test_a_cache_that_does_not_fit_is_refused(what, own_gemm):
