@@ -779,6 +779,7 @@ __device__ __forceinline__ void select_body(const SelectParams& p) {
   const int C = p.cluster;
   int pair = blockIdx.x / C;  // (sequence, kv head); re-mapped below when the grid runs in several waves
   const int crank = blockIdx.x - pair * C;  // rank inside the cluster that shares this pair
+  if (C > 1) cluster_arrive_started();
   // Launched with programmatic dependent launch: nothing in global memory may be read
   // before the predecessor on the stream has completed (it may have produced the
   // lengths or the query, and the attention kernel of the previous step may still be
@@ -1348,6 +1349,7 @@ __device__ __forceinline__ void select_body(const SelectParams& p) {
     }
   }
   __syncthreads();
+  if (C > 1) cluster_wait_started();  // the peers run: their shared memory may be written (a rank without tiles is here early)
   IA_TRACE(4);
 
   // ---- phase 2: merge the warps' row normalisers (warp g merges row g as a tree) ---------

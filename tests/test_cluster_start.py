@@ -25,6 +25,8 @@ def _body(file, signature):
 
 @pytest.mark.parametrize("file,signature,remote_store", [
     ("llama_step.cu", "llama_argmax_parts_kernel(const PartsView", "st.shared::cluster"),
+    ("select_kernel.cuh", "select_body(const SelectParams& p)", "st_cluster_f32("),
+    ("select_kernel.cuh", "select_body(const SelectParams& p)", "map_to_rank("),
 ])
 def test_no_remote_store_before_the_whole_cluster_runs(file, signature, remote_store):
     body = _body(file, signature)
