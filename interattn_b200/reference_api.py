@@ -98,6 +98,14 @@ class _PrefixHandle:
         self.c_summ = summ.c_struct()
         self.geom_flags = ops._geom_flags(summ) | _lib.IA_GEOM_SUFFIX_LENS
 
+    def __getstate__(self):
+        """A prefix may be copied or saved: the addresses stay behind, a copy has its own."""
+        return {name: value for name, value in self.__dict__.items() if name != "c_summ"}
+
+    def __setstate__(self, state):
+        self.__dict__.update(state)
+        self.c_summ = self.summ.c_struct()
+
 
 def _stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)

@@ -263,6 +263,31 @@ def test_suffix_length_read_on_the_device(dtype, d, suffix_len):
     assert torch.equal(got, again)
 
 
+def test_a_copied_prefix_decodes_after_the_original_is_gone():
+    """The copy addresses its own summaries, lengths and table: the original's memory is released and overwritten."""
+    import copy
+    api = _api()
+    hkv, g, d, block, prompt = 2, 4, 128, 64, 700
+    k, v = (x.to(DEV) for x in _cache(hkv, prompt, d, torch.bfloat16, 19))
+    q = torch.randn((hkv, g, 1, d), generator=torch.Generator().manual_seed(6)).to(torch.bfloat16).to(DEV)
+    length = torch.zeros((), dtype=torch.int32, device=DEV)
+
+    def decode(prefix):
+        return api._condition_block_decode_output_fused_triton(
+            q_grouped=q, prompt_prefix=prefix, k_suffix=k[:, prompt:], v_suffix=v[:, prompt:], suffix_len_dev=length,
+            eps=None, top_k=3, page_size=block, store_selected=False, output_dtype=None, workspace={}, kv_cache=(k, v))[0]
+
+    prefix = api._build_prompt_blocks(k, v, block)
+    want = decode(prefix).clone()
+    other = copy.deepcopy(prefix)
+    h = prefix["_b200"]
+    for t in (h.summ.k_bar, h.summ.k_max, h.summ.k_min, h.summ.v_bar, h.summ.v_norm_max):
+        t.fill_(float("nan"))
+    h.geometry.table.fill_(0)
+    del prefix, h, t
+    assert torch.equal(decode(other), want)
+
+
 def test_fused_decode_topk_and_workspace_reuse():
     api = _api()
     hkv, g, d, block, prompt_len = 2, 8, 128, 64, 2000

@@ -1,6 +1,9 @@
 """Host-side behaviour of the reference-named calls, without a GPU: tensors that only claim to be on one (fake
 tensors), and a library that records its calls instead of launching anything."""
 
+import copy
+import io
+
 import pytest
 import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
@@ -35,3 +38,28 @@ def test_the_suffix_length_lives_on_the_cache_device():
                 api._condition_block_decode_output_fused_triton(
                     q_grouped=q, prompt_prefix=prefix, k_suffix=empty, v_suffix=empty, suffix_len_dev=length, eps=None,
                     top_k=1, page_size=BLOCK, store_selected=False, output_dtype=None, workspace={})
+
+
+def _pointers(struct):
+    return [getattr(struct, name) for name, _ in struct._fields_]
+
+
+@pytest.mark.parametrize("how", ["copy", "deepcopy", "save"])
+def test_a_prefix_can_be_copied_and_saved(how):
+    """The handle keeps the summaries' addresses in the form the library takes; a copy has those of its own tensors."""
+    prefix = _prefix("cpu")
+    prefix["_b200"].summ.v_bar.fill_(3.0)
+    if how == "save":
+        buf = io.BytesIO()
+        torch.save(prefix, buf)
+        buf.seek(0)
+        other = torch.load(buf, weights_only=False)
+    else:
+        other = getattr(copy, how)(prefix)
+        if how == "copy":
+            other["_b200"] = copy.copy(prefix["_b200"])
+    h = other["_b200"]
+    assert _pointers(h.c_summ) == _pointers(h.summ.c_struct())
+    assert (_pointers(h.c_summ) == _pointers(prefix["_b200"].c_summ)) == (how == "copy")
+    assert torch.equal(h.summ.v_bar, prefix["_b200"].summ.v_bar)
+    assert (h.block_size, h.prompt_len, h.geom_flags) == (BLOCK, PROMPT, prefix["_b200"].geom_flags)
