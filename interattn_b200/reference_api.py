@@ -31,6 +31,7 @@ from typing import Dict, Optional, Tuple
 
 import torch
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from . import _lib, ops
 from ._lib import Geom, IA_REP_HYBRID, IA_REP_SPARSE_ONLY, IA_SELECT_EPS, IA_SELECT_TOPK, check
@@ -144,8 +145,9 @@ def _build_prompt_blocks(k_all: torch.Tensor, v_all: torch.Tensor, block_size: i
     packed = os.environ.get("CONDITION_BLOCK_TMA_BOUNDS") == "1"
     mixed = os.environ.get("CONDITION_BLOCK_MIXED_SUMMARIES") == "1"
     pad = nb * block_size - length
-    # A copy that autograd should follow (the cache is part of a graph) is made by torch, below.
-    own_copy = pad > 0 and not (torch.is_grad_enabled() and (k_all.requires_grad or v_all.requires_grad))
+    # A copy that autograd should follow (the cache is part of a graph, or carries a tangent) is made by torch, below.
+    own_copy = pad > 0 and not (torch.is_grad_enabled() and (k_all.requires_grad or v_all.requires_grad)) \
+        and forward_ad.unpack_dual(k_all).tangent is None and forward_ad.unpack_dual(v_all).tangent is None
     copies = 0 if mixed or k_all.dtype == torch.float32 else 1 if packed else 3   # fp32 copies: v_bar, k_max, k_min
 
     # One launch writes all of it (an empty prompt is refused there).

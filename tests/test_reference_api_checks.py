@@ -63,3 +63,47 @@ def test_a_prefix_can_be_copied_and_saved(how):
     assert (_pointers(h.c_summ) == _pointers(prefix["_b200"].c_summ)) == (how == "copy")
     assert torch.equal(h.summ.v_bar, prefix["_b200"].summ.v_bar)
     assert (h.block_size, h.prompt_len, h.geom_flags) == (BLOCK, PROMPT, prefix["_b200"].geom_flags)
+
+
+class _Library:
+    """Takes any call and remembers its name."""
+
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        def call(*args):
+            self.calls.append(name)
+            return 0
+        return call
+
+
+@pytest.fixture
+def recorder(monkeypatch):
+    lib = _Library()
+    monkeypatch.setattr(api._lib, "load", lambda: lib)
+    monkeypatch.setattr(api, "_stream", lambda: None)
+    return lib
+
+
+@pytest.mark.filterwarnings("ignore:Accessing the data pointer")
+@pytest.mark.parametrize("length", [PROMPT - 1, PROMPT])
+@pytest.mark.parametrize("which", ["k", "v"])
+def test_blocked_copies_carry_a_tangent(length, which, recorder):
+    """Forward-mode differentiation goes through k_block_attn / v_block_attn, padded copies or views alike."""
+    from torch.autograd import forward_ad
+    with FakeTensorMode(), forward_ad.dual_level():
+        k, v = (torch.empty((HKV, length, D), dtype=torch.bfloat16, device="cuda:0") for _ in range(2))
+        dual = forward_ad.make_dual(k if which == "k" else v, torch.empty_like(k))
+        prefix = api._build_prompt_blocks(dual if which == "k" else k, dual if which == "v" else v, BLOCK)
+        assert recorder.calls == ["ia_build_prompt_blocks"]
+        for name in ("k", "v"):
+            tangent = forward_ad.unpack_dual(prefix[f"{name}_block_attn"]).tangent
+            assert (tangent is not None) == (name == which), name
+
+
+@pytest.mark.filterwarnings("ignore:Accessing the data pointer")
+def test_blocked_copies_of_a_cache_with_gradients(recorder):
+    with FakeTensorMode():
+        k, v = (torch.empty((HKV, PROMPT - 1, D), dtype=torch.bfloat16, device="cuda:0") for _ in range(2))
+        assert api._build_prompt_blocks(k, v.requires_grad_(), BLOCK)["v_block_attn"].requires_grad
