@@ -150,20 +150,22 @@ def _build_prompt_blocks(k_all: torch.Tensor, v_all: torch.Tensor, block_size: i
         and forward_ad.unpack_dual(k_all).tangent is None and forward_ad.unpack_dual(v_all).tangent is None
     copies = 0 if mixed or k_all.dtype == torch.float32 else 1 if packed else 3   # fp32 copies: v_bar, k_max, k_min
 
-    # One launch writes all of it (an empty prompt is refused there).
+    # One launch writes all of it (an empty prompt is refused there).  Every array has a storage of its own: a caller
+    # may keep, save or change one without the others.
     new, slab = k_all.new_empty, (1, hkv, nb, d)
     k_bar = new(slab, dtype=getattr(torch, k_bar_name))
-    v_bar, k_max, k_min = new((3, *slab)).unbind(0)
+    v_bar = new(slab)
     v_norm_max, v_norm_all = new((1, hkv, nb), dtype=torch.float32), new((hkv,), dtype=torch.float32)
     token_idx, counts = new((nb, block_size), dtype=torch.int64), new((nb,), dtype=torch.int64)
     valid_token = new((nb, block_size), dtype=torch.bool)
-    f32 = new((copies, hkv, nb, d), dtype=torch.float32).unbind(0) if copies else ()
-    blocks = new((2, hkv, nb, block_size, d)).unbind(0) if own_copy else ()
-    k_bounds = None
-    if packed:   # the space of the two bound arrays as one array of pairs
-        k_bounds = k_max.as_strided((1, hkv, nb, 2 * d), (hkv * nb * 2 * d, nb * 2 * d, 2 * d, 1))
+    f32 = [new(slab[1:], dtype=torch.float32) for _ in range(copies)]
+    blocks = [new((hkv, nb, block_size, d)) for _ in range(2 if own_copy else 0)]
+    if packed:
+        k_bounds = new((1, hkv, nb, 2 * d))
         pairs = k_bounds.view(1, hkv, nb, d, 2)
         k_max, k_min = pairs[..., 0], pairs[..., 1]
+    else:
+        k_bounds, k_max, k_min = None, new(slab), new(slab)
     summ = ops.BlockSummaries(k_bar=k_bar, k_max=k_max, k_min=k_min, v_bar=v_bar, v_norm_max=v_norm_max,
                               block_size=block_size, k_bounds=k_bounds)
     geometry = _CacheGeometry(dev, length)

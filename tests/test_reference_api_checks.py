@@ -107,3 +107,27 @@ def test_blocked_copies_of_a_cache_with_gradients(recorder):
     with FakeTensorMode():
         k, v = (torch.empty((HKV, PROMPT - 1, D), dtype=torch.bfloat16, device="cuda:0") for _ in range(2))
         assert api._build_prompt_blocks(k, v.requires_grad_(), BLOCK)["v_block_attn"].requires_grad
+
+
+@pytest.mark.parametrize("mixed", ["0", "1"])
+@pytest.mark.parametrize("packed", ["0", "1"])
+@pytest.mark.filterwarnings("ignore:Accessing the data pointer")
+def test_every_array_of_a_prefix_has_its_own_storage(packed, mixed, recorder, monkeypatch):
+    """Keeping, saving or changing one of them does not keep, save or touch another (the views into the packed
+    range apart)."""
+    monkeypatch.setenv("CONDITION_BLOCK_TMA_BOUNDS", packed)
+    monkeypatch.setenv("CONDITION_BLOCK_MIXED_SUMMARIES", mixed)
+    with FakeTensorMode():
+        k, v = (torch.empty((HKV, PROMPT - 1, D), dtype=torch.bfloat16, device="cuda:0") for _ in range(2))
+        prefix = api._build_prompt_blocks(k, v, BLOCK)
+    views = {"k_max", "k_min"} if packed == "1" else set()
+    for name, t in prefix.items():
+        if torch.is_tensor(t) and name not in views:
+            assert t.untyped_storage().nbytes() == t.numel() * t.element_size(), name
+            assert t.is_contiguous() and (t._base is None or t._base.numel() == t.numel()), name
+    h = prefix["_b200"]
+    stored = [h.summ.k_bar, h.summ.v_bar, h.summ.v_norm_max] + ([h.summ.k_bounds] if views else [h.summ.k_max, h.summ.k_min])
+    assert all(t.untyped_storage().nbytes() == t.numel() * t.element_size() for t in stored)
+    if views:
+        assert all(getattr(h.summ, n).shape == (1, HKV, NB, D) and getattr(h.summ, n).stride(3) == 2 for n in views)
+        assert h.summ.k_min.storage_offset() == h.summ.k_bounds.storage_offset() + 1
