@@ -85,10 +85,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     if (mbar_test(bar, parity)) return true;
   return false;
 }
+__device__ __forceinline__ unsigned long long global_timer_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
 // The same for waits that take microseconds and whose end nothing urgent follows: try_wait parks the warp, which
-// leaves its scheduler to the warps that issue copies and MMAs.
+// leaves its scheduler to the warps that issue copies and MMAs.  How long one try_wait parks is up to the hardware, so
+// this wait is bounded by the clock.
+constexpr unsigned long long kParkedWaitNs = 1000000000ull;
 __device__ __forceinline__ bool mbar_wait_parked(uint64_t* bar, uint32_t parity) {
-  for (uint32_t i = 0; i < kWaitPolls; ++i) {
+  const unsigned long long start = global_timer_ns();
+  do {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -98,7 +106,7 @@ __device__ __forceinline__ bool mbar_wait_parked(uint64_t* bar, uint32_t parity)
         : "r"(smem_u32(bar)), "r"(parity)
         : "memory");
     if (ok != 0) return true;
-  }
+  } while (global_timer_ns() - start < kParkedWaitNs);
   return false;
 }
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -535,12 +543,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) llama_stream_gemm_kernel(const 
         load_x(n, x.kc, stage_base + (size_t)i * R::stage_bytes, &full_bar[i]);
         x.advance(n);
       }
-      bool alive = true;
       int stage = 0, parity = 0;  // of the empty barrier: use u of a stage waits for the release of use u - 1
-      for (; !w.done();) {
-        if (alive && !mbar_wait(&empty_bar[stage], (uint32_t)parity)) {
-          alive = false;
+      int issued = primed;
+      for (; !w.done(); ++issued) {
+        if (!mbar_wait(&empty_bar[stage], (uint32_t)parity)) {  // the MMA thread has given up
           atomicOr(p.status, DEV_STATUS_GEMM_WAIT_TIMEOUT);
+          break;
         }
         const int n = w.template len<CPS>();
         unsigned char* st = stage_base + (size_t)stage * R::stage_bytes;
@@ -550,10 +558,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) llama_stream_gemm_kernel(const 
         step_w(n);
         if (++stage == kStages) { stage = 0; parity ^= 1; }
       }
+      // the last copy into each stage has landed before the CTA ends, also when nobody consumes it any more
+      for (int s = 0; s < kStages && s < issued; ++s)
+        if (!mbar_wait(&full_bar[s], (uint32_t)(((issued - 1 - s) / kStages) & 1))) {
+          atomicOr(p.status, DEV_STATUS_GEMM_WAIT_TIMEOUT);
+          break;
+        }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      bool alive = true;
+      grid_dependency_wait();  // no x before that: the bounded waits below are for this kernel's copies alone
+      int last_stage = -1, last_parity = 0;
       int seg = 0, stage = 0, parity = 0;
       StageWalk m(c0, c1, KC);
       while (!m.done()) {
@@ -561,16 +576,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) llama_stream_gemm_kernel(const 
         const bool first = m.starts_tile_or_range(c0);
         if (first) {
           const int buf = seg & 1, use = seg >> 1;
-          if (use > 0 && alive && !mbar_wait(&acc_empty[buf], (uint32_t)((use - 1) & 1))) {
-            alive = false;
+          if (use > 0 && !mbar_wait(&acc_empty[buf], (uint32_t)((use - 1) & 1))) {
             atomicOr(p.status, DEV_STATUS_GEMM_WAIT_TIMEOUT);
+            break;
           }
           ++seg;
         }
         const int buf = (seg - 1) & 1;
-        if (alive && !mbar_wait(&full_bar[stage], (uint32_t)parity)) {
-          alive = false;
+        if (!mbar_wait(&full_bar[stage], (uint32_t)parity)) {
           atomicOr(p.status, DEV_STATUS_GEMM_WAIT_TIMEOUT);
+          break;
         }
         tc_fence_after();
         const uint32_t st = smem_u32(stage_base + (size_t)stage * R::stage_bytes);
@@ -585,10 +600,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) llama_stream_gemm_kernel(const 
           b_desc += R::chunk_x >> 4;
         }
         umma_commit(&empty_bar[stage]);
+        last_stage = stage;
+        last_parity = parity;
         m.advance(n);
         if (m.kc == 0 || m.done()) umma_commit(&acc_full[buf]);
         if (++stage == kStages) { stage = 0; parity ^= 1; }
       }
+      // given up: the MMAs issued so far end before the tensor memory is returned (else the epilogue has seen to that)
+      if (!m.done() && last_stage >= 0) mbar_wait(&empty_bar[last_stage], (uint32_t)last_parity);
     }
   } else {
     grid_dependency_wait();  // the slots and the output may still be read by earlier kernels
