@@ -103,6 +103,45 @@ def test_fused_step_head_dim_64(cfg, shape, cluster, rep_mode, monkeypatch):
     test_fused_step_matches_selection_and_oracle(cfg, shape, cluster, rep_mode, monkeypatch)
 
 
+STORAGES = {"packed": dict(packed_bounds=True), "diag_ell": dict(diag_ell=True), "kbar16": dict(k_bar_dtype=torch.bfloat16),
+            "kbar16_packed": dict(k_bar_dtype=torch.bfloat16, packed_bounds=True),
+            "kbar16_diag_ell": dict(k_bar_dtype=torch.bfloat16, diag_ell=True)}
+
+
+@pytest.mark.parametrize("rep_mode", ["sparse_only", "hybrid"])
+@pytest.mark.parametrize("shape,cluster", [("wide", 2), ("narrow", 2)])
+@pytest.mark.parametrize("storage", list(STORAGES))
+@pytest.mark.parametrize("cfg", D64_CASES, ids=lambda c: c.name)
+def test_fused_step_head_dim_64_summary_storages(cfg, storage, shape, cluster, rep_mode, monkeypatch):
+    """The other forms of the summaries have kernels (and shared-memory layouts) of their own: each must run as one
+    kernel, pick what the stand-alone selection picks and attend over exactly that, as the two-kernel form does."""
+    ops = _ops()
+    monkeypatch.setenv("INTERATTN_B200_SELECT_CLUSTER", str(cluster))
+    monkeypatch.setenv("INTERATTN_B200_SELECT_SHAPE", shape)
+    case = make_case(cfg, spare_pages=3)
+    q, kv = to_device(case)
+    summ = ops.build_summaries(kv, cfg.block_size, max_blocks=max_blocks_of(case), **STORAGES[storage])
+    kw = dict(top_k=cfg.top_k, bound="diag_ell" if "diag_ell" in storage else "range")
+    step = ops.DecodeAttention(kv, summ, cfg.n_q_heads, rep_mode=rep_mode, **kw)
+    for _ in range(2):
+        out = step.step(q).clone()
+        assert ops.last_decode_fused(), "the pinned shape must take the one-kernel form"
+    idx, cnt, aux = ops.select_blocks(q, summ, kv.prefix_lens, want=("z",), **kw)
+    two_step = ops.DecodeAttention(kv, summ, cfg.n_q_heads, rep_mode=rep_mode, **kw)
+    before = ops.set_fused_step(False)
+    try:
+        two = two_step.step(q).clone()
+        assert not ops.last_decode_fused()
+    finally:
+        ops.set_fused_step(before)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    for s in (step, two_step):
+        assert torch.equal(s.sel_idx[:, :, :idx.shape[2]], idx) and torch.equal(s.sel_count, cnt)
+    _check_against_oracle(cfg, case, summ, out, idx, cnt, rep_mode, aux["z"])
+    torch.testing.assert_close(out.float(), two.float(), **TOL)
+
+
 def test_switch_between_the_one_kernel_and_the_two_kernel_form(monkeypatch):
     ops = _ops()
     monkeypatch.setenv("INTERATTN_B200_SELECT_CLUSTER", "1")
