@@ -158,14 +158,20 @@ def _build_prompt_blocks(k_all: torch.Tensor, v_all: torch.Tensor, block_size: i
     v_norm_max, v_norm_all = new((1, hkv, nb), dtype=torch.float32), new((hkv,), dtype=torch.float32)
     token_idx, counts = new((nb, block_size), dtype=torch.int64), new((nb,), dtype=torch.int64)
     valid_token = new((nb, block_size), dtype=torch.bool)
-    f32 = [new(slab[1:], dtype=torch.float32) for _ in range(copies)]
-    blocks = [new((hkv, nb, block_size, d)) for _ in range(2 if own_copy else 0)]
+    like = torch.empty_like   # 1.0 us of host time instead of 1.7
+    f32, blocks, k_bounds = [], [], None
+    if copies:
+        f32.append(new(slab[1:], dtype=torch.float32))
+        f32.extend(like(f32[0]) for _ in range(copies - 1))
+    if own_copy:
+        blocks.append(new((hkv, nb, block_size, d)))
+        blocks.append(like(blocks[0]))
     if packed:
         k_bounds = new((1, hkv, nb, 2 * d))
         pairs = k_bounds.view(1, hkv, nb, d, 2)
         k_max, k_min = pairs[..., 0], pairs[..., 1]
     else:
-        k_bounds, k_max, k_min = None, new(slab), new(slab)
+        k_max, k_min = like(v_bar), like(v_bar)
     summ = ops.BlockSummaries(k_bar=k_bar, k_max=k_max, k_min=k_min, v_bar=v_bar, v_norm_max=v_norm_max,
                               block_size=block_size, k_bounds=k_bounds)
     geometry = _CacheGeometry(dev, length)
