@@ -495,6 +495,7 @@ int ia_llama_gemm(const void* x, const void* w_packed, void* out, int m, int n, 
  * bf16 and goes on as its namesake above does on the finished projection.  x, w: 16-byte aligned, k a multiple of 8,
  * m <= 16.  `out` (bf16 [m, n], else null): tiles that one CTA summed alone are written there instead, finished;
  * ia_llama_argmax_parts completes the others.
+ * w is read while the kernel in front of this one on the stream may still run: that kernel must not write it.
  *   add_rmsnorm_parts: n = hidden (a multiple of 8)
  *   rope_append_parts: n = (n_q_heads + 2 n_kv_heads) * head_dim, head_dim a multiple of 8; tables, caches and q_out
  *                      8-byte aligned

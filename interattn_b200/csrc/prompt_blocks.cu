@@ -36,9 +36,9 @@ struct PromptParams {
 // per lane in flight), the launch for short ones.  A token row is read by D sizeof(T) / 16 lanes with 16 bytes each,
 // so one warp load covers 2 tokens (head_dim 128 bf16) and a lane owns eight coordinates; the paged kernels'
 // 8-byte lanes need twice the instructions, and their persistent 14-warp CTAs cover a 4099-token prompt
-// (520 blocks) with 38 of the 148 SMs.  8 heads, 4099 tokens, head_dim 128 bf16: 6.8 us for all outputs, where the
-// paged kernel took 13.2 us for the summaries alone and 23 small launches made the rest; the whole call 219 -> 82 us,
-// most of it now the host's allocation of the output tensors.
+// (520 blocks) with 38 of the 148 SMs.  8 heads, 4099 tokens, head_dim 128 bf16: 6.7 us for all outputs, where the
+// paged kernel took 13.2 us for the summaries alone and 23 small launches made the rest; the whole call 206 - 219 ->
+// 77 us, most of it now the host's allocation of the output tensors.
 template <typename T, int D>
 __global__ void __launch_bounds__(kThreads) condition_block_prompt_blocks_kernel(const __grid_constant__ PromptParams<T> p) {
   constexpr int VEC = 16 / (int)sizeof(T);  // coordinates per lane

@@ -24,8 +24,8 @@ constexpr int kWarps = 4;
 // each step serves the 16 tokens together: one exchange joins a token's two half dots, the maximum takes four
 // exchanges per query row, and the weights reach the lanes of the V product through shared memory.  One token after
 // the other (a warp reduction and an exponential chain each) took 0.3 us per token.  Two fp32 sequences of 1024
-// tokens, 4 pairs x 16 pages, head_dim 64:
-// 19.7 -> 8.1 us, the step 29.4 -> 16.5 us (it also overlaps the selection kernel's end now, by programmatic launch).
+// tokens, 4 pairs x 16 pages, head_dim 64: 19.7 -> 8.1 us, the step 28.7 -> 15.4 us (it also
+// overlaps the selection kernel's end now, by programmatic launch).
 template <typename T, int D, int G>
 __global__ void __launch_bounds__(kWarps * 32)
 condition_block_finalize_attention_fma_kernel(const __grid_constant__ DecodeParams p) {
